@@ -991,13 +991,6 @@ int launch_potential(const Dev& d, const Cfg& c, cudaStream_t s) {
   return 1;
 }
 
-// Gravity only (group MAC), for point sets without SPH.
-int launch_gravity_group(const Dev& d, const Cfg& c, cudaStream_t s) {
-  if (c.quad) walk<4, true, true, false, false, kWalkAccPhi>(d, c, s);
-  else walk<4, true, false, false, false, kWalkAccPhi>(d, c, s);
-  return 1;
-}
-
 // Neighbour lists only (when gravity is not the tree).
 int launch_neighbours(const Dev& d, const Cfg& c, cudaStream_t s) {
   walk<4, false, false, true, false, kWalkAcc>(d, c, s);

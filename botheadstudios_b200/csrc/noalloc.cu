@@ -262,7 +262,7 @@ extern "C" sph_status sph_gravity_tree_noalloc(const void* d_bodies4, uint32_t n
   launch_bbox(d, s);
   launch_sort_permute(d, s);
   launch_tree(d, c, theta, s);
-  launch_gravity_group(d, c, s);
+  launch_gravity_points(d, c, s);
   k_noalloc_store<<<(n + 255) / 256, 256, 0, s>>>((int)n, d.s().id, d.grav, d.P, static_cast<float4*>(d_acc4));
   // no error was pending on entry, so one pending now comes from these launches: report it (and clear it)
   return cudaGetLastError() == cudaSuccess ? SPH_OK : SPH_ERR_CUDA;

@@ -1212,7 +1212,7 @@ sph_status sph_gravity(sph_ctx* ctx, const double* pos3, const double* mass, uin
   launch_sort_permute(g, s);
   if (gravity_mode == SPH_GRAVITY_TREE) {
     launch_tree(g, ctx->kc, ctx->cfg.theta, s);
-    if (ctx->kc.mac == SPH_MAC_GROUP) launch_gravity_group(g, ctx->kc, s);
+    if (ctx->kc.mac == SPH_MAC_GROUP) launch_gravity_points(g, ctx->kc, s);
     else launch_gravity_tree(g, ctx->kc, s);
   } else {
     launch_gravity_direct(g, s);

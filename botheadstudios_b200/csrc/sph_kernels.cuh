@@ -249,7 +249,7 @@ int launch_neighbours(const Dev& d, const Cfg& c, cudaStream_t s);      // neigh
 // group-MAC gravity + neighbour lists; potential: also the potential φ (the steps' walks leave it out)
 int launch_walk(const Dev& d, const Cfg& c, bool potential, cudaStream_t s);
 int launch_potential(const Dev& d, const Cfg& c, cudaStream_t s);      // φ alone on the current tree
-int launch_gravity_group(const Dev& d, const Cfg& c, cudaStream_t s);   // group-MAC gravity only
+int launch_gravity_points(const Dev& d, const Cfg& c, cudaStream_t s);  // gravity of a point set without SPH (h = 0)
 int launch_density_eos(const Dev& d, const Cfg& c, cudaStream_t s);
 int launch_h_solve(const Dev& d, const Cfg& c, cudaStream_t s);
 int launch_h_learned(const Dev& d, const Cfg& c, cudaStream_t s);   // check proposals, iterate the rejected
