@@ -39,8 +39,7 @@ struct DiskWork {
   void* base = nullptr;
   unsigned long long* keys[2] = {nullptr, nullptr};
   unsigned* vals[2] = {nullptr, nullptr};
-  unsigned* hist = nullptr;
-  unsigned* tot = nullptr;
+  void* sort_work = nullptr;
   double* part = nullptr;   // [kDmBlocks][kDmVals] block partials
   double* tsum = nullptr;   // [tiles] mass of each radius-sorted tile
   double* scal = nullptr;   // [S_COUNT]
@@ -78,7 +77,7 @@ constexpr int kDmThreads = 256;
 constexpr int kDmBlocks = 592;  // 4 × 148 SMs; block b reduces the b-th contiguous chunk of the impact
 constexpr int kDmVals = 8;
 constexpr int kPeRows = 128;    // particles per self-potential row
-constexpr int kTile = 2048;     // radius-sorted tile of the crossing walk (the radix sort's tile)
+constexpr int kTile = 2048;     // radius-sorted tile of the crossing walk
 constexpr unsigned kCellBias = 1u << 20, kCellMax = (1u << 21) - 1u;
 constexpr int kUnionTries = 1 << 16;
 constexpr unsigned long long kMaxUnits = 1ull << 28;  // self-potential tile pairs (2 GB of partial sums)
@@ -957,12 +956,12 @@ int bits_of(unsigned v) {
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Carve the workspace for m particles from one allocation.
-bool work_reserve(DiskWork* w, int m) {
+bool work_reserve(DiskWork* w, int m, cudaStream_t s) {
   if (w->cap >= m && w->base) return true;
   if (w->base) cudaFree(w->base);
   w->base = nullptr;
   w->cap = 0;
-  const size_t n = (size_t)(m < 1 ? 1 : m), half = n / 2 + 2, tiles = radix_tiles((int)n);
+  const size_t n = (size_t)(m < 1 ? 1 : m), half = n / 2 + 2, tiles = (n + kTile - 1) / kTile;
   size_t sz = 0;
   auto take = [&](size_t bytes) {
     const size_t o = sz;
@@ -970,7 +969,7 @@ bool work_reserve(DiskWork* w, int m) {
     return o;
   };
   const size_t o_k0 = take(8 * n), o_k1 = take(8 * n), o_v0 = take(4 * n), o_v1 = take(4 * n);
-  const size_t o_hist = take(4 * 256 * tiles), o_tot = take(4 * 256), o_part = take(8 * kDmBlocks * kDmVals);
+  const size_t o_sort = take(sort_work_bytes((int)n)), o_part = take(8 * kDmBlocks * kDmVals);
   const size_t o_tsum = take(8 * tiles), o_scal = take(8 * S_COUNT), o_cnt = take(4 * C_COUNT);
   const size_t o_bcnt = take(4 * kDmBlocks), o_cat = take(n);
   const size_t o_pm = take(16 * n), o_p0 = take(16 * n), o_p1 = take(16 * n), o_u0 = take(16 * n), o_u1 = take(16 * n);
@@ -979,6 +978,10 @@ bool work_reserve(DiskWork* w, int m) {
   const size_t o_out = take(8 * 16), o_bb = take(8 * 16), o_pl = take(8 * 12 * kMaxPlacements);
   void* base = nullptr;
   if (cudaMalloc(&base, sz) != cudaSuccess) return false;
+  if (cudaMemsetAsync((char*)base + o_sort, 0, sort_work_bytes((int)n), s) != cudaSuccess) {
+    cudaFree(base);
+    return false;
+  }
   char* b = (char*)base;
   w->base = base;
   w->cap = (int)n;
@@ -986,8 +989,7 @@ bool work_reserve(DiskWork* w, int m) {
   w->keys[1] = (unsigned long long*)(b + o_k1);
   w->vals[0] = (unsigned*)(b + o_v0);
   w->vals[1] = (unsigned*)(b + o_v1);
-  w->hist = (unsigned*)(b + o_hist);
-  w->tot = (unsigned*)(b + o_tot);
+  w->sort_work = b + o_sort;
   w->part = (double*)(b + o_part);
   w->tsum = (double*)(b + o_tsum);
   w->scal = (double*)(b + o_scal);
@@ -1018,7 +1020,7 @@ int launch_radius_crossing(DiskWork* w, const float4* pm, unsigned n, const doub
                            double frac, double* out, cudaStream_t s) {
   k_dm_radius<<<(n + 255) / 256, 256, 0, s>>>(pm, n, centre, w->keys[0], w->vals[0]);
   int src = 0;
-  int L = 1 + launch_radix_sort(w->keys, w->vals, (int)n, 64, w->hist, w->tot, src, s);
+  int L = 1 + launch_radix_sort(w->keys, w->vals, (int)n, 64, w->sort_work, w->cnt + C_ERR, src, s);
   const int tiles = (int)((n + kTile - 1) / kTile);
   k_dm_tile_mass<<<tiles, kDmThreads, 0, s>>>(pm, n, w->vals[src], w->tsum);
   k_dm_cross<<<1, 1024, 0, s>>>(pm, n, tiles, w->keys[src], w->vals[src], w->tsum, total, frac, out);
@@ -1040,7 +1042,7 @@ int disk_measure(const Dev& d, unsigned off, unsigned m, const DiskCfg& c, DiskW
   *launches = 0;
   if (m == 0) return 0;
   if (!w) w = new DiskWork();
-  if (!work_reserve(w, (int)m)) {
+  if (!work_reserve(w, (int)m, s)) {
     *err = "disk measure: workspace allocation failed";
     return -3;
   }
@@ -1068,7 +1070,7 @@ int disk_measure(const Dev& d, unsigned off, unsigned m, const DiskCfg& c, DiskW
     k_dm_compact<<<nb, kDmThreads, 0, s>>>(st, d.rho, off, m, chunk, w->cat, w->bcnt, w->scal, w->dpos[0],
                                            w->dvel[0], w->drp[0], w->keys[0], w->vals[0]);
     L += 1;
-    L += launch_radix_sort(w->keys, w->vals, (int)nd, 63, w->hist, w->tot, src, s);
+    L += launch_radix_sort(w->keys, w->vals, (int)nd, 63, w->sort_work, w->cnt + C_ERR, src, s);
     const unsigned gb = (nd + 255) / 256;
     k_dm_gather<<<gb, 256, 0, s>>>(nd, w->vals[src], w->dpos[0], w->dvel[0], w->drp[0], w->dpos[1], w->dvel[1],
                                    w->drp[1], w->parent, w->gcnt);
@@ -1077,7 +1079,7 @@ int disk_measure(const Dev& d, unsigned off, unsigned m, const DiskCfg& c, DiskW
                                                              w->parent, w->cnt);
     k_dm_roots<<<gb, 256, 0, s>>>(nd, w->parent, w->gcnt, w->keys[0], w->vals[0]);
     L += 3;
-    L += launch_radix_sort(w->keys, w->vals, (int)nd, bits_of(nd), w->hist, w->tot, src, s);
+    L += launch_radix_sort(w->keys, w->vals, (int)nd, bits_of(nd), w->sort_work, w->cnt + C_ERR, src, s);
     k_dm_gather<<<gb, 256, 0, s>>>(nd, w->vals[src], w->dpos[1], w->dvel[1], w->drp[1], w->dpos[0], w->dvel[0],
                                    w->drp[0], nullptr, nullptr);
     k_dm_clumps<<<gb, 256, 0, s>>>(nd, w->keys[src], w->gcnt, w->clump, w->cnt);
@@ -1130,6 +1132,10 @@ int disk_measure(const Dev& d, unsigned off, unsigned m, const DiskCfg& c, DiskW
     return -2;
   }
   *launches = L;
+  if (flags[C_ERR] & kFlagSortTimeout) {
+    *err = "disk measure: a sort's waits ran out";
+    return -4;
+  }
   if (flags[C_ERR]) {
     *err = "disk measure: a union-find hook gave up after its retry limit";
     return -5;
@@ -1140,9 +1146,9 @@ int disk_measure(const Dev& d, unsigned off, unsigned m, const DiskCfg& c, DiskW
 
 namespace {
 
-int reserve_or_fail(DiskWork*& w, unsigned m, const char** err) {
+int reserve_or_fail(DiskWork*& w, unsigned m, const char** err, cudaStream_t s) {
   if (!w) w = new DiskWork();
-  if (!work_reserve(w, (int)(m ? m : 1u))) {
+  if (!work_reserve(w, (int)(m ? m : 1u), s)) {
     *err = "body measurement: workspace allocation failed";
     return -3;
   }
@@ -1199,7 +1205,7 @@ int body_bulk(const Dev& d, unsigned prov, DiskWork*& w, double* out5, unsigned 
   *launches = 0;
   for (int k = 0; k < 5; ++k) out5[k] = 0.0;
   if (d.n == 0) return 0;
-  if (int rc = reserve_or_fail(w, (unsigned)d.n, err)) return rc;
+  if (int rc = reserve_or_fail(w, (unsigned)d.n, err, s)) return rc;
   return body_bulk_impl(d, prov, w, out5, launches, err, s);
 }
 
@@ -1214,7 +1220,7 @@ int assemble_n(const Dev& d, const double* placements, unsigned np, void* dst, u
   }
   const unsigned n = (unsigned)d.n;
   if (n == 0 || np == 0) return 0;
-  if (int rc = reserve_or_fail(w, n, err)) return rc;
+  if (int rc = reserve_or_fail(w, n, err, s)) return rc;
   unsigned long long L = 0;
   double place[kMaxPlacements * 12];
   for (unsigned k = 0; k < np; ++k) {

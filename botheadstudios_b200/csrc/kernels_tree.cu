@@ -1,5 +1,5 @@
-// LBVH construction on B200: bounding box → 30-bit Morton keys → LSD radix sort → state permutation →
-// Karras internal nodes → single-pass bottom-up moments.
+// LBVH construction on B200: bounding box → 30-bit Morton keys → LSD radix sort (kernels_sort.cu) → state
+// permutation → Karras internal nodes → single-pass bottom-up moments.
 //
 // Reference: shaders/bh_gravity.wgsl (cs_bbox :68, cs_morton :100, cs_tree :135, cs_com :201) and the CPU
 // sort of crates/engine/src/gpu_gravity.rs:336-368. The sort order is (Morton code, original index), made
@@ -93,170 +93,10 @@ __global__ void k_bbox(const float4* __restrict__ pos, const unsigned* __restric
   seg_bbox_commit(lo, hi, sg, segs);
 }
 
-int launch_bbox(const Dev& d, cudaStream_t s) {
+static int launch_bbox(const Dev& d, cudaStream_t s) {
   k_bbox_reset<<<1, kMaxSegments, 0, s>>>(d.segs, d.nseg);
   k_bbox<<<(d.n + 255) / 256, 256, 0, s>>>(d.s().pos_h, d.s().seg, d.n, d.segs);
   return 2;
-}
-
-// ---------------------------------------------------------------------------------------------------
-// Morton keys (cs_morton, bh_gravity.wgsl:91-108) with IEEE division, no contraction, each particle
-// quantised in its own segment's box. The sort order is (segment, code, original index): each key
-// segment << 30 | code is written at its particle's original index, so a stable sort on the key alone leaves
-// equal keys in index order (30 + segment bits instead of 30 + segment + index bits: 4 passes, not 7, at 1M).
-// ---------------------------------------------------------------------------------------------------
-__global__ void k_keys(const float4* __restrict__ pos, const unsigned* __restrict__ id,
-                       const unsigned* __restrict__ seg, int n, const Seg* __restrict__ segs,
-                       unsigned long long* __restrict__ keys, unsigned* __restrict__ vals) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const unsigned sg = seg[i];
-  const unsigned* bb = segs[sg].bbox;
-  float lo[3], ext[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    lo[k] = key_float(bb[k]);
-    ext[k] = fmaxf(fsub(key_float(bb[3 + k]), lo[k]), 1.0e-30f);
-  }
-  const float4 p = pos[i];
-  const float pc[3] = {p.x, p.y, p.z};
-  unsigned q[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    float u = fdiv(fsub(pc[k], lo[k]), ext[k]);
-    u = fminf(fmaxf(u, 0.0f), 1.0f);
-    float f = floorf(fmul(u, 1024.0f));
-    f = fminf(fmaxf(f, 0.0f), 1023.0f);
-    q[k] = (unsigned)f;
-  }
-  const unsigned code = expand_bits(q[0]) * 4u + expand_bits(q[1]) * 2u + expand_bits(q[2]);
-  const unsigned o = id[i];  // a permutation of [0, n)
-  keys[o] = ((unsigned long long)sg << 30) | code;
-  vals[o] = (unsigned)i;
-}
-
-// ---------------------------------------------------------------------------------------------------
-// LSD radix sort, 8-bit digits, reduce-then-scan (no inter-block waits): upsweep histograms per tile,
-// per-digit scans over tiles, stable downsweep (warp match_any ranking, staged through shared memory).
-// ---------------------------------------------------------------------------------------------------
-constexpr int RS_THREADS = 256;
-constexpr int RS_ITEMS = 8;
-constexpr int RS_TILE = RS_THREADS * RS_ITEMS;  // 2048 keys per tile
-constexpr int RS_WARPS = RS_THREADS / 32;
-
-size_t radix_tiles(int n) { return (size_t)((n + RS_TILE - 1) / RS_TILE); }
-
-__global__ void __launch_bounds__(RS_THREADS) k_rs_upsweep(const unsigned long long* __restrict__ keys, int n,
-                                                           int shift, unsigned* __restrict__ hist, int T) {
-  __shared__ unsigned h[256];
-  h[threadIdx.x] = 0;
-  __syncthreads();
-  const int base = blockIdx.x * RS_TILE;
-#pragma unroll
-  for (int it = 0; it < RS_ITEMS; ++it) {
-    const int idx = base + it * RS_THREADS + threadIdx.x;
-    if (idx < n) atomicAdd(&h[(unsigned)(keys[idx] >> shift) & 255u], 1u);
-  }
-  __syncthreads();
-  hist[threadIdx.x * T + blockIdx.x] = h[threadIdx.x];
-}
-
-// One block per digit: exclusive scan of hist[d][0..T) in place; tot[d] = sum.
-__global__ void __launch_bounds__(1024) k_rs_scan(unsigned* __restrict__ hist, unsigned* __restrict__ tot, int T) {
-  __shared__ unsigned s_warp[33];
-  unsigned* h = hist + (size_t)blockIdx.x * T;
-  const int per = (T + blockDim.x - 1) / blockDim.x;
-  const int b0 = threadIdx.x * per;
-  unsigned sum = 0;
-  for (int i = 0; i < per; ++i)
-    if (b0 + i < T) sum += h[b0 + i];
-  unsigned total;
-  unsigned run = block_exclusive_scan(sum, s_warp, total);
-  for (int i = 0; i < per; ++i)
-    if (b0 + i < T) {
-      const unsigned v = h[b0 + i];
-      h[b0 + i] = run;
-      run += v;
-    }
-  if (threadIdx.x == 0) tot[blockIdx.x] = total;
-}
-
-__global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(const unsigned long long* __restrict__ kin,
-                                                             const unsigned* __restrict__ vin,
-                                                             unsigned long long* __restrict__ kout,
-                                                             unsigned* __restrict__ vout, int n, int shift,
-                                                             const unsigned* __restrict__ hist,
-                                                             const unsigned* __restrict__ tot, int T) {
-  __shared__ unsigned long long s_keys[RS_TILE];
-  __shared__ unsigned s_vals[RS_TILE];
-  __shared__ unsigned s_wcnt[RS_WARPS][256];
-  __shared__ unsigned s_gbin[256];     // global output start of digit d for this tile
-  __shared__ unsigned s_bstart[256];   // start of digit d inside the tile
-  __shared__ unsigned s_warp[33];
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int base = blockIdx.x * RS_TILE;
-
-  // global digit starts: exclusive scan of the digit totals + this tile's prefix
-  unsigned total;
-  const unsigned dstart = block_exclusive_scan(tot[tid], s_warp, total);
-  s_gbin[tid] = dstart + hist[tid * T + blockIdx.x];
-#pragma unroll
-  for (int k = 0; k < RS_WARPS; ++k) s_wcnt[k][tid] = 0;
-  __syncthreads();
-
-  unsigned long long key[RS_ITEMS];
-  unsigned val[RS_ITEMS], dig[RS_ITEMS], loc[RS_ITEMS];
-  const unsigned lt_mask = (1u << lane) - 1u;
-#pragma unroll
-  for (int it = 0; it < RS_ITEMS; ++it) {
-    const int idx = base + (w * RS_ITEMS + it) * 32 + lane;
-    const bool ok = idx < n;
-    key[it] = ok ? kin[idx] : 0ull;
-    val[it] = ok ? vin[idx] : 0u;
-    const unsigned d = ok ? ((unsigned)(key[it] >> shift) & 255u) : 256u;
-    dig[it] = d;
-    const unsigned peers = __match_any_sync(SPH_FULL_MASK, d);
-    const int leader = __ffs(peers) - 1;
-    unsigned old = 0;
-    if (lane == leader && ok) {
-      old = s_wcnt[w][d];
-      s_wcnt[w][d] = old + __popc(peers);
-    }
-    old = __shfl_sync(SPH_FULL_MASK, old, leader);
-    loc[it] = old + __popc(peers & lt_mask);
-    __syncwarp();
-  }
-  __syncthreads();
-  // per digit: exclusive prefix over warps, then over digits within the tile
-  {
-    unsigned run = 0;
-#pragma unroll
-    for (int k = 0; k < RS_WARPS; ++k) {
-      const unsigned c = s_wcnt[k][tid];
-      s_wcnt[k][tid] = run;
-      run += c;
-    }
-    unsigned t2;
-    s_bstart[tid] = block_exclusive_scan(run, s_warp, t2);
-  }
-  __syncthreads();
-#pragma unroll
-  for (int it = 0; it < RS_ITEMS; ++it) {
-    if (dig[it] < 256u) {
-      const unsigned p = s_bstart[dig[it]] + s_wcnt[w][dig[it]] + loc[it];
-      s_keys[p] = key[it];
-      s_vals[p] = val[it];
-    }
-  }
-  __syncthreads();
-  const int cnt = min(RS_TILE, n - base);
-  for (int i = tid; i < cnt; i += RS_THREADS) {
-    const unsigned long long k = s_keys[i];
-    const unsigned d = (unsigned)(k >> shift) & 255u;
-    const unsigned g = s_gbin[d] + (unsigned)i - s_bstart[d];
-    kout[g] = k;
-    vout[g] = s_vals[i];
-  }
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -285,50 +125,21 @@ __global__ void k_permute(int n, int L, const unsigned* __restrict__ order,
   if (t < L) leaf_codes[t] = skeys[leaf_start[t]];
 }
 
-int launch_sort_permute(Dev& d, cudaStream_t s) {
+// The sort order is (segment, code, original index): the sort is stable and starts out in original-index order
+// (kernels_sort.cu). Each particle is quantised in its own segment's box.
+int launch_sort_permute(Dev& d, bool need_bbox, cudaStream_t s) {
   const int n = d.n;
-  const int threads = 256;
-  const int blocks = (n + threads - 1) / threads;
+  const int box = need_bbox ? launch_bbox(d, s) : 0;
   const State& in = d.st[d.cur];
-  k_keys<<<blocks, threads, 0, s>>>(in.pos_h, in.id, in.seg, n, d.segs, d.keys[0], d.vals[0]);
-  const int T = (int)radix_tiles(n);
-  const int total_bits = 30 + d.segbits;
-  const int passes = (total_bits + 7) / 8;
-  int src = 0;
-  for (int shift = 0; shift < total_bits; shift += 8) {
-    k_rs_upsweep<<<T, RS_THREADS, 0, s>>>(d.keys[src], n, shift, d.rs_hist, T);
-    k_rs_scan<<<256, 1024, 0, s>>>(d.rs_hist, d.rs_tot, T);
-    k_rs_downsweep<<<T, RS_THREADS, 0, s>>>(d.keys[src], d.vals[src], d.keys[src ^ 1], d.vals[src ^ 1], n, shift,
-                                             d.rs_hist, d.rs_tot, T);
-    src ^= 1;
-  }
-  // vals[src] = old slot of each sorted position; keys[src] = sorted keys
   const State& out = d.st[d.cur ^ 1];
-  k_permute<<<blocks, threads, 0, s>>>(n, d.L, d.vals[src], d.keys[src], d.leaf_start, in, out, d.body,
-                                       d.leaf_codes);
+  int src = 0;
+  const int sorts = launch_morton_sort(d, src, s);
+  // vals[src] = old slot of each sorted position; keys[src] = sorted keys
+  k_permute<<<(n + 255) / 256, 256, 0, s>>>(n, d.L, d.vals[src], d.keys[src], d.leaf_start, in, out, d.body,
+                                            d.leaf_codes);
   d.cur ^= 1;
-  // keep the sorted keys in keys[0] for inspection
-  if (src != 0) cudaMemcpyAsync(d.keys[0], d.keys[src], sizeof(unsigned long long) * n, cudaMemcpyDeviceToDevice, s);
-  return 2 + 3 * passes;
-}
-
-// Stable LSD radix sort of n (key, value) pairs on the low `bits` key bits, ping-ponging between buf 0 and 1.
-// Returns the buffer holding the result in `src`; hist holds 256 × radix_tiles(n) counters.
-int launch_radix_sort(unsigned long long* keys[2], unsigned* vals[2], int n, int bits, unsigned* hist,
-                      unsigned* tot, int& src, cudaStream_t s) {
-  src = 0;
-  if (n <= 1) return 0;
-  const int T = (int)radix_tiles(n);
-  int launches = 0;
-  for (int shift = 0; shift < bits; shift += 8) {
-    k_rs_upsweep<<<T, RS_THREADS, 0, s>>>(keys[src], n, shift, hist, T);
-    k_rs_scan<<<256, 1024, 0, s>>>(hist, tot, T);
-    k_rs_downsweep<<<T, RS_THREADS, 0, s>>>(keys[src], vals[src], keys[src ^ 1], vals[src ^ 1], n, shift, hist,
-                                             tot, T);
-    src ^= 1;
-    launches += 3;
-  }
-  return launches;
+  d.sorted = src;
+  return box + sorts + 1;
 }
 
 // ---------------------------------------------------------------------------------------------------

@@ -23,6 +23,7 @@ namespace {
 constexpr uint32_t kNoAllocMaxPoints = 65536;
 constexpr uint32_t kNoAllocMinLeaf = 8;  // bounds the node arrays: at most kNoAllocMaxPoints / 8 leaves
 constexpr size_t kAlign = 256;
+constexpr size_t kNoAllocSort = kSortCtlBytes + kNoAllocMaxPoints / kSortTileMin * kSortTileBytes;  // the sort's workspace
 
 constexpr size_t up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 
@@ -31,12 +32,11 @@ constexpr size_t scratch_bytes() {
   const size_t n = kNoAllocMaxPoints;
   const size_t L = n / kNoAllocMinLeaf;
   const size_t nodes = 2 * L;
-  const size_t tiles = (n + 2047) / 2048;
   size_t b = 0;
   b += 2 * (up(16 * n) + up(16 * n) + 3 * up(8 * n) + 5 * up(4 * n));  // two particle states
   b += 2 * up(8 * n) + 2 * up(4 * n);                                  // sort keys and values
   b += up(16 * n) + up(16 * n);                                        // bodies, accelerations
-  b += up(4 * 256 * tiles) + up(4 * 256);                              // radix histograms
+  b += up(kNoAllocSort);                                               // the sort's workspace
   b += up(8 * L) + 3 * up(4 * L) + up(8 * L) + up(4);                  // leaf codes, left/right/counters, groups
   b += up(4 * (L + 1)) + up(2 * sizeof(Seg));                          // leaf starts, segment table
   b += up(4 * nodes) + 5 * up(16 * nodes);                             // parents, node records
@@ -163,9 +163,7 @@ Dev carve_dev(unsigned char* base, uint32_t K) {
   d.vals[1] = carve<unsigned>(p, n);
   d.body = carve<float4>(p, n);
   d.grav = carve<float4>(p, n);
-  d.rs_tiles_cap = (int)((n + 2047) / 2048);
-  d.rs_hist = carve<unsigned>(p, 256 * (size_t)d.rs_tiles_cap);
-  d.rs_tot = carve<unsigned>(p, 256);
+  d.sort_work = carve<unsigned char>(p, kNoAllocSort);  // zero when the library is loaded
   d.leaf_codes = carve<unsigned long long>(p, L);
   d.left = carve<unsigned>(p, L);
   d.right = carve<unsigned>(p, L);
@@ -259,8 +257,7 @@ extern "C" sph_status sph_gravity_tree_noalloc(const void* d_bodies4, uint32_t n
   k_noalloc_params<<<1, 1, 0, s>>>(d.P, (float)G, theta);
   k_noalloc_load<<<(n + 255) / 256, 256, 0, s>>>(static_cast<const float4*>(d_bodies4), (int)n, d.st[0]);
   launch_segments_single(d, softening * softening, 0.0, s);
-  launch_bbox(d, s);
-  launch_sort_permute(d, s);
+  launch_sort_permute(d, true, s);
   launch_tree(d, c, theta, s);
   launch_gravity_points(d, c, s);
   k_noalloc_store<<<(n + 255) / 256, 256, 0, s>>>((int)n, d.s().id, d.grav, d.P, static_cast<float4*>(d_acc4));

@@ -120,9 +120,10 @@ sph_status alloc_dev(sph_ctx* ctx, Dev& d, uint32_t cap, uint32_t K, uint32_t nb
     ALLOC(d.vals[b], capw);
   }
   ALLOC(d.body, capw);
-  d.rs_tiles_cap = (int)radix_tiles((int)cap);
-  ALLOC(d.rs_hist, 256 * (size_t)(d.rs_tiles_cap > 0 ? d.rs_tiles_cap : 1));
-  ALLOC(d.rs_tot, 256);
+  unsigned char* sort_work = nullptr;
+  ALLOC(sort_work, sort_work_bytes((int)cap));
+  CK(cudaMemsetAsync(sort_work, 0, sort_work_bytes((int)cap), ctx->stream));
+  d.sort_work = sort_work;
   ALLOC(d.leaf_codes, Lmax);
   ALLOC(d.leaf_start, Lmax + 1);
   ALLOC(d.segs, (size_t)kMaxSegments + 1);
@@ -243,7 +244,7 @@ sph_status rebuild(sph_ctx* ctx, bool need_bbox, bool potential) {
   Dev& d = ctx->d;
   cudaStream_t s = ctx->stream;
   const Cfg& c = ctx->kc;
-  phase(ctx, SPH_PHASE_SORT, [&] { return (need_bbox ? launch_bbox(d, s) : 0) + launch_sort_permute(d, s); });
+  phase(ctx, SPH_PHASE_SORT, [&] { return launch_sort_permute(d, need_bbox, s); });
   phase(ctx, SPH_PHASE_TREE, [&] { return launch_tree(d, c, ctx->cfg.theta, s); });
   const bool fused = fused_walk(ctx);
   ctx->evaluated = true;
@@ -965,6 +966,10 @@ sph_status sph_diag(sph_ctx* ctx, sph_diag_out* out) {
   out->p2p_interactions = p.stat_p2p;
   out->local_expansions = p.stat_m2l;
   out->p2p_slots = p.stat_p2p_slots;
+  if (p.flags & kFlagSortTimeout) {
+    ctx->err = "the Morton sort's waits ran out";
+    return SPH_ERR_TIMEOUT;
+  }
   if (p.flags & (kFlagNbrOverflow | kFlagStackOverflow)) {
     ctx->err = "device capacity overflow (flags " + std::to_string(p.flags) + ")";
     return SPH_ERR_OVERFLOW;
@@ -1015,7 +1020,7 @@ sph_status sph_inspect(sph_ctx* ctx, uint32_t what, void* host_out, size_t bytes
     case SPH_Q_CODES: {
       if (!need(n * 4)) return SPH_ERR_INVALID;
       std::vector<unsigned long long> k(n);
-      CK(cudaMemcpy(k.data(), d.keys[0], n * 8, cudaMemcpyDeviceToHost));
+      CK(cudaMemcpy(k.data(), d.keys[d.sorted], n * 8, cudaMemcpyDeviceToHost));
       for (size_t t = 0; t < n; ++t) ((unsigned*)host_out)[t] = (unsigned)(k[t] & 0x3fffffffu);
       return SPH_OK;
     }
@@ -1208,8 +1213,7 @@ sph_status sph_gravity(sph_ctx* ctx, const double* pos3, const double* mass, uin
   DevParams p = ctx->hp;
   CK(cudaMemcpyAsync(g.P, &p, sizeof(p), cudaMemcpyHostToDevice, s));
   launch_segments_single(g, (float)softening * (float)softening, 0.0, s);
-  launch_bbox(g, s);
-  launch_sort_permute(g, s);
+  launch_sort_permute(g, true, s);
   if (gravity_mode == SPH_GRAVITY_TREE) {
     launch_tree(g, ctx->kc, ctx->cfg.theta, s);
     if (ctx->kc.mac == SPH_MAC_GROUP) launch_gravity_points(g, ctx->kc, s);
@@ -1483,7 +1487,7 @@ sph_status sph_dem_step(sph_dem* dem, uint32_t substeps) {
   Dev& d = ctx->d;
   cudaStream_t s = ctx->stream;
   for (uint32_t k = 0; k < substeps; ++k) {
-    phase(ctx, SPH_PHASE_SORT, [&] { return launch_bbox(d, s) + launch_sort_permute(d, s); });
+    phase(ctx, SPH_PHASE_SORT, [&] { return launch_sort_permute(d, true, s); });
     phase(ctx, SPH_PHASE_TREE, [&] { return launch_tree(d, ctx->kc, ctx->cfg.theta, s); });
     phase(ctx, SPH_PHASE_NEIGHBOURS, [&] { return launch_neighbours(d, ctx->kc, s); });
     phase(ctx, SPH_PHASE_FORCES, [&] { return launch_dem_contacts(d, dem->p, dem->acc, s); });

@@ -14,7 +14,8 @@ constexpr int kTravStack = 64;      // bh_gravity.wgsl:336 MAX_STACK
 constexpr float kPiF = 3.14159265359f;  // sph_step.wgsl:20
 
 // Device-side error/overflow flags (bit set, never cleared by kernels).
-enum : unsigned { kFlagNbrOverflow = 1u, kFlagStackOverflow = 2u, kFlagCandOverflow = 4u, kFlagTensorTimeout = 8u };
+enum : unsigned { kFlagNbrOverflow = 1u, kFlagStackOverflow = 2u, kFlagCandOverflow = 4u, kFlagTensorTimeout = 8u,
+                kFlagSortTimeout = 16u };
 
 // Material row as in SphEos48 (Tillotson, 12 floats).
 struct Eos {
@@ -120,6 +121,22 @@ __device__ __forceinline__ unsigned expand_bits(unsigned v) {
   v = (v * 0x00000011u) & 0xc30c30c3u;
   v = (v * 0x00000005u) & 0x49249249u;
   return v;
+}
+
+// The 30-bit Morton code of a position in its impact's box (cs_morton, bh_gravity.wgsl:91-108): IEEE division, no
+// contraction. ext: the box's extents, floored at 1e-30.
+__device__ __forceinline__ unsigned morton_code(float4 p, const float lo[3], const float ext[3]) {
+  const float pc[3] = {p.x, p.y, p.z};
+  unsigned q[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    float u = fdiv(fsub(pc[k], lo[k]), ext[k]);
+    u = fminf(fmaxf(u, 0.0f), 1.0f);
+    float f = floorf(fmul(u, 1024.0f));
+    f = fminf(fmaxf(f, 0.0f), 1023.0f);
+    q[k] = (unsigned)f;
+  }
+  return expand_bits(q[0]) * 4u + expand_bits(q[1]) * 2u + expand_bits(q[2]);
 }
 
 // ---- SPH kernels with support radius h: the reference's cubic spline (sph_step.wgsl:64-77) and Wendland C2 --

@@ -140,9 +140,8 @@ struct Dev {
   float4* body = nullptr;  // x, y, z, m in sorted order (gravity sources)
   unsigned long long* keys[2] = {nullptr, nullptr};
   unsigned* vals[2] = {nullptr, nullptr};
-  unsigned* rs_hist = nullptr;  // [256][tiles]
-  unsigned* rs_tot = nullptr;   // [256]
-  int rs_tiles_cap = 0;
+  void* sort_work = nullptr;    // the sort's control block and published tile counts (sort_work_bytes)
+  int sorted = 0;               // the keys/vals buffer that holds the last sort's result
   int nseg = 1;
   int segbits = 0;                 // sort-key bits of the segment index (0 for one segment)
   Seg* segs = nullptr;             // [kMaxSegments + 1]
@@ -228,15 +227,20 @@ int launch_dem_integrate(const Dev& d, const DemParams& p, const float4* acc, cu
 // ---- segments and tree -----------------------------------------------------------------------------
 int launch_segments(const Dev& d, cudaStream_t s);        // leaf_start from the segment table
 int launch_segments_single(const Dev& d, float soft2, double dt, cudaStream_t s);  // one segment, on the device
-int launch_bbox(const Dev& d, cudaStream_t s);
-int launch_sort_permute(Dev& d, cudaStream_t s);      // keys → radix sort → permute (swaps d.cur)
+// keys → radix sort → permute (swaps d.cur); need_bbox: the bounding boxes first
+int launch_sort_permute(Dev& d, bool need_bbox, cudaStream_t s);
 int launch_tree(const Dev& d, const Cfg& c, float theta, cudaStream_t s);  // Karras + moments
 // particles per half leaf the group walk splits far leaves into (0: leaves are not split)
 int half_leaf(const Dev& d, const Cfg& c);
-size_t radix_tiles(int n);
-// stable LSD radix sort of (keys, vals) on the low `bits` key bits; the result lands in buffer `src`
-int launch_radix_sort(unsigned long long* keys[2], unsigned* vals[2], int n, int bits, unsigned* hist,
-                      unsigned* tot, int& src, cudaStream_t s);
+// Stable LSD radix sort (kernels_sort.cu) on the low `bits` key bits; the result lands in buffer `src`. `work`:
+// sort_work_bytes(n) of device memory, zero before its first sort and used by one sort at a time; a sort whose
+// waits run out raises kFlagSortTimeout in *flags.
+constexpr size_t kSortCtlBytes = 32768, kSortTileBytes = 8192, kSortTileMin = 1024;
+size_t sort_work_bytes(int n);
+int launch_radix_sort(unsigned long long* const keys[2], unsigned* const vals[2], int n, int bits, void* work,
+                      unsigned* flags, int& src, cudaStream_t s);
+// Morton keys of the current state (segment << 30 | code), sorted with the particles' slots
+int launch_morton_sort(const Dev& d, int& src, cudaStream_t s);
 
 // ---- gravity ---------------------------------------------------------------------------------------
 int launch_gravity_tree(const Dev& d, const Cfg& c, cudaStream_t s);
