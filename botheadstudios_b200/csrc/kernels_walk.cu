@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
     const float4* __restrict__ ncom, const float4* __restrict__ nbmin, const float4* __restrict__ nbmax, const float4* __restrict__ nq0,
     const float4* __restrict__ nq1, DevParams* P, float4* __restrict__ gout, unsigned* __restrict__ nbr,
     unsigned* __restrict__ nbr_cnt, unsigned cap, float skin, float* __restrict__ h0,
-    const uint2* __restrict__ groups, const unsigned* __restrict__ ngroups, int stack_cap, float local_theta,
+    const uint2* __restrict__ groups, int ngroups, int stack_cap, float local_theta,
     int half, const float4* __restrict__ hcom, const float4* __restrict__ hq0, const float2* __restrict__ hq1,
     const float2* __restrict__ hrc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
   const int w = threadIdx.x >> 5;
   const unsigned lane = threadIdx.x & 31u;
   const int warp = blockIdx.x * W + w;
-  if (warp >= (int)*ngroups) return;
+  if (warp >= ngroups) return;
   // this warp's group: a run of <= 32 Morton-consecutive particles of one impact (leaves g.x..g.y); the walk
   // starts at that impact's root
   const uint2 grp = groups[warp];
@@ -939,8 +939,7 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
 
 template <int W, bool GRAV, bool QUAD, bool NBR, bool HILO, int OUT>
 static void walk(const Dev& d, const Cfg& c, cudaStream_t s) {
-  const int warps = d.L;  // upper bound on the number of groups
-  const int blocks = (warps + W - 1) / W;
+  const int blocks = (d.ngroups + W - 1) / W;
   const size_t smem = sizeof(WalkSmem<W>);
   static std::atomic<unsigned long long> attr{0};
   smem_limit_per_device(k_tree_walk<W, GRAV, QUAD, NBR, HILO, OUT>, (int)smem, attr);

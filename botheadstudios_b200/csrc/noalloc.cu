@@ -37,7 +37,7 @@ constexpr size_t scratch_bytes() {
   b += 2 * up(8 * n) + 2 * up(4 * n);                                  // sort keys and values
   b += up(16 * n) + up(16 * n);                                        // bodies, accelerations
   b += up(kNoAllocSort);                                               // the sort's workspace
-  b += up(8 * L) + 3 * up(4 * L) + up(8 * L) + up(4);                  // leaf codes, left/right/counters, groups
+  b += 2 * up(8 * L) + 2 * up(4 * L) + up(8 * L);                      // leaf codes, slots, left/right, groups
   b += up(4 * (L + 1)) + up(2 * sizeof(Seg));                          // leaf starts, segment table
   b += up(4 * nodes) + 5 * up(16 * nodes);                             // parents, node records
   b += 2 * up(16 * L) + 2 * up(8 * L);                                 // half-leaf moments (leaves of >= 16)
@@ -167,9 +167,8 @@ Dev carve_dev(unsigned char* base, uint32_t K) {
   d.leaf_codes = carve<unsigned long long>(p, L);
   d.left = carve<unsigned>(p, L);
   d.right = carve<unsigned>(p, L);
-  d.counters = carve<unsigned>(p, L);
+  d.slots = carve<unsigned long long>(p, L);  // zero when the library is loaded
   d.groups = carve<uint2>(p, L);
-  d.ngroups = carve<unsigned>(p, 1);
   d.leaf_start = carve<unsigned>(p, L + 1);
   d.segs = carve<Seg>(p, 2);
   d.parent = carve<unsigned>(p, nodes);

@@ -131,6 +131,8 @@ sph_status alloc_dev(sph_ctx* ctx, Dev& d, uint32_t cap, uint32_t K, uint32_t nb
   ALLOC(d.right, Lmax);
   ALLOC(d.parent, nodes);
   ALLOC(d.counters, Lmax);
+  ALLOC(d.slots, Lmax);
+  CK(cudaMemsetAsync(d.slots, 0, Lmax * sizeof(*d.slots), ctx->stream));
   ALLOC(d.ncom, nodes);
   ALLOC(d.nbmin, nodes);
   ALLOC(d.nbmax, nodes);
@@ -142,7 +144,6 @@ sph_status alloc_dev(sph_ctx* ctx, Dev& d, uint32_t cap, uint32_t K, uint32_t nb
   ALLOC(d.hrc, Lmax);
   ALLOC(d.grav, capw);
   ALLOC(d.groups, Lmax);
-  ALLOC(d.ngroups, 1);
   ALLOC(d.P, 1);
   if (sph) {
     d.nbr_cap = nbr_cap;
@@ -335,20 +336,27 @@ sph_status upload_impl(sph_ctx* ctx, const SphParticle48* particles, const uint3
   d.segbits = nimp > 1 ? bits_for(nimp) : 0;
   // segment table: each impact's leaves are K-particle buckets from its first particle
   std::vector<Seg> table((size_t)d.nseg + 1);
-  uint32_t L = 0;
+  uint32_t L = 0, groups = 0;
+  const uint32_t per = (uint32_t)group_leaves(d.K);
   for (uint32_t k = 0; k <= nimp; ++k) {
     Seg& g = table[k];
     std::memset(&g, 0, sizeof(g));
     g.off = k < nimp ? off[k] : nu;
     g.loff = L;
+    g.pad = groups;
     g.sig_bits = 0x7f800000u;
     for (int a = 0; a < 3; ++a) g.bbox[a] = 0xffffffffu;
     g.soft2 = k < nimp ? soft[k] * soft[k] : 0.0f;
     g.skin = ctx->hp.skin_wide;  // new positions: the first rebuild's solve gets the wide skin
     g.dt = ctx->hp.dt_fixed;
-    if (k < nimp) L += (off[k + 1] - off[k] + (uint32_t)d.K - 1) / (uint32_t)d.K;
+    if (k < nimp) {
+      const uint32_t leaves = (off[k + 1] - off[k] + (uint32_t)d.K - 1) / (uint32_t)d.K;
+      L += leaves;
+      groups += (leaves + per - 1) / per;
+    }
   }
   d.L = (int)L;
+  d.ngroups = (int)groups;
   ctx->n_eos = ne;
   if (!keep_eos) {
     Eos etab[kMaxMaterials];
@@ -1462,6 +1470,7 @@ sph_status sph_dem_replace(sph_dem* dem, const SphGrain80* grains, uint32_t n) {
   d.n = (int)n;
   d.cur = 0;
   d.L = n ? (int)((n + d.K - 1) / d.K) : 0;
+  d.ngroups = (d.L + group_leaves(d.K) - 1) / group_leaves(d.K);
   d.nseg = 1;
   d.segbits = 0;
   dem->stepped = false;

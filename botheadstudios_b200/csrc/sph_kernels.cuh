@@ -47,7 +47,7 @@ struct Seg {
   unsigned sig_bits;    // atomicMin target: bits of the segment's minimum Courant signal
   unsigned bbox[6];     // order-preserving keys of lo.xyz, hi.xyz (bh_gravity.wgsl:49-57)
   float soft2;          // softening² of this impact
-  unsigned pad;         // first walk group of the impact
+  unsigned pad;         // first walk group of the impact (host-written with the table)
   unsigned res_bits;    // atomicMax target: the impact's smoothing-length residual maximum (float bits)
   float skin;           // neighbour-list skin of the impact's next rebuild (smoothing-length solve)
   double dt;            // dt of the current step
@@ -150,7 +150,8 @@ struct Dev {
   unsigned* left = nullptr;     // [L-1]
   unsigned* right = nullptr;    // [L-1]
   unsigned* parent = nullptr;   // [2L-1]
-  unsigned* counters = nullptr; // [L-1] climb arrival counters
+  unsigned* counters = nullptr; // [L-1] climb arrival counters (per-particle walk)
+  unsigned long long* slots = nullptr;  // [L-1] meeting places of siblings (group walk); zero between builds
   float4* ncom = nullptr;       // [2L-1] com.xyz, mass
   float4* nbmin = nullptr;      // [2L-1] bmin.xyz, max h
   float4* nbmax = nullptr;      // [2L-1] bmax.xyz, opening radius
@@ -163,7 +164,7 @@ struct Dev {
   float2* hq1 = nullptr;        // [2L] Qxz, Qyz
   float2* hrc = nullptr;        // [L] opening radii of the two halves (size/θ + |centre − COM|)
   uint2* groups = nullptr;      // [L] walk groups: (first leaf, last leaf) of runs of 32/K leaves of one impact
-  unsigned* ngroups = nullptr;  // [1] number of groups
+  int ngroups = 0;              // number of groups
   unsigned* nbr = nullptr;      // interleaved neighbour lists [n/32][nbr_cap][32]
   unsigned* nbr_cnt = nullptr;  // [n]
   unsigned nbr_cap = 0;
@@ -225,11 +226,12 @@ int launch_dem_contacts(const Dev& d, const DemParams& p, float4* acc, cudaStrea
 int launch_dem_integrate(const Dev& d, const DemParams& p, const float4* acc, cudaStream_t s);
 
 // ---- segments and tree -----------------------------------------------------------------------------
-int launch_segments(const Dev& d, cudaStream_t s);        // leaf_start from the segment table
+constexpr int group_leaves(int K) { return 32 / K; }      // leaves of a walk group
+int launch_segments(const Dev& d, cudaStream_t s);        // leaf starts and walk groups from the segment table
 int launch_segments_single(const Dev& d, float soft2, double dt, cudaStream_t s);  // one segment, on the device
 // keys → radix sort → permute (swaps d.cur); need_bbox: the bounding boxes first
 int launch_sort_permute(Dev& d, bool need_bbox, cudaStream_t s);
-int launch_tree(const Dev& d, const Cfg& c, float theta, cudaStream_t s);  // Karras + moments
+int launch_tree(const Dev& d, const Cfg& c, float theta, cudaStream_t s);  // links + moments
 // particles per half leaf the group walk splits far leaves into (0: leaves are not split)
 int half_leaf(const Dev& d, const Cfg& c);
 // Stable LSD radix sort (kernels_sort.cu) on the low `bits` key bits; the result lands in buffer `src`. `work`:
