@@ -1,18 +1,19 @@
 // Fused LBVH group walk: Barnes-Hut gravity (group MAC, monopole + optional quadrupole) and the SPH
-// neighbour lists in ONE traversal per warp.
+// neighbour lists in ONE traversal per group.
 //
-// A warp owns 32 Morton-consecutive particles (its "group") and walks the tree with a LIFO stack in shared
-// memory, popping up to 32 nodes at a time (one per lane) so node loads overlap instead of serialising.
+// A group is a run of 32 Morton-consecutive particles, lane l of every warp that walks for it holding particle l. The
+// walk keeps a LIFO stack in shared memory and pops up to 32 nodes for each of its warps at a time (one per lane) so
+// node loads overlap instead of serialising.
 // Each popped node is classified for the whole group:
 //   * accepted  — the MAC sqrt(d²+ε²) >= side/θ + |centre−COM| (the node's largest side, as the reference's
 //                 CPU octree measures it, bhtree.rs:181, with the δ term of bh_gravity.wgsl:382) holds for the
 //                 nearest point of the group's bounding box, hence for every particle of the group, and the
 //                 node's box is outside the SPH reach: appended to the multipole list;
-//   * leaf      — appended to the near list (pairwise gravity + the neighbour test) when some particle of the
-//                 group can reach it with its own smoothing length (a per-lane test after the group test),
-//                 otherwise to the far list (pairwise gravity only); with half leaves a far leaf is queued, and
-//                 a later pass classifies the halves of up to 32 queued leaves at once (each half a multipole,
-//                 a term of the group's local expansion, or 8 pairwise sources);
+//   * leaf      — appended to the near list (pairwise gravity + the neighbour test) when the group can reach it (with
+//                 leaves of 16 and more: when some particle can, with its own smoothing length, a per-lane test after
+//                 the group test), otherwise to the far list (pairwise gravity only); with half leaves a far leaf is
+//                 queued, and a later round classifies the halves of up to 32 queued leaves a warp (each half a
+//                 multipole, a term of the group's local expansion, or 8 pairwise sources);
 //   * opened    — children pushed (ballot + popc compaction).
 // Accepted nodes far from the group (beyond r_group/θ_L) go into the group's local expansion instead of the
 // per-particle multipole list.
@@ -25,29 +26,54 @@
 // The interaction loops take the staged sources two at a time with the packed FP32x2 add/multiply/fma of sm_100
 // (each half rounded as the scalar operation); their reciprocal square roots are the bare special-function
 // operation.
+//
+// How many warps walk for a group depends on its impact's size alone (an impact of a batch gets the sums it would get
+// alone). One warp is the cheapest: nothing to wait for, bound by instruction issue. But an impact of 10,240 particles
+// is 320 groups on 592 schedulers, and its walk lasts as long as one group's chain of pops and flushes. So up to
+// kSharedWalkMax particles four warps share a group's stack and lists, in rounds: 10,240 particles 0.14 ms (one warp
+// 0.51), 32,768 0.21 (0.40), 65,536 0.38 (0.54). With three contexts stepping at once, so that other groups fill the
+// schedulers, a step of 20,000 particles takes 136 µs with four warps and 180 with one, 45,000 291 and 307, 65,536 434
+// and 406, 100,000 668 and 598: the line lies below the size where they cross, for batches of many impacts.
+//
+// Near pairs. The neighbour test of a source is the sign of d² − lim², shifted into a mask of the chunk (one
+// instruction each), and a lane writes its finds after the chunk; the particle itself needs no test (its force is a
+// finite number times zero). 22 instructions for a pair of sources instead of about 40. With the local expansion's sums
+// kept in registers over a list of 448 nodes instead of 32 (one transposed sum for each flush) the walk went from 5.95
+// to 5.01 ms at 1,048,576 particles and from 25.9 to 22.7 ms at 4,194,304.
 #include <type_traits>
 
 #include "sph_kernels.cuh"
 
 namespace sphb {
 
-constexpr int TW_STACK = 1280;  // per-warp node stack
-constexpr int TW_LIST = 96;     // per-warp list capacity (a pop adds <= 64 entries; flushed above 32)
-constexpr int TW_WARPS_PER_SM = 24;  // resident walk warps per SM (80 registers, ~8.4 KB shared each)
+// Resident walk warps per SM (72 registers; 8.6 KB of shared memory for a warp of its own). At 1,048,576 particles 24
+// warps took 5.14 ms, 26 5.01, 28 5.02, 30 (64 registers, spilled) 5.03.
+constexpr int TW_WARPS_PER_SM = 26;
 
-// Per-block shared memory of a W-warp walk block (the traversal tile: W groups of 32 particles).
-template <int W>
+// Shared memory of a block of F warps that walk for one group of 32 particles. A round of nodes adds at most 32 F
+// entries to a list, a round of halves 64 F (two per lane); lists are flushed when a round might not fit.
+template <int F>
 struct WalkSmem {
-  unsigned stack[W][TW_STACK];
-  unsigned m2p[W][TW_LIST];
-  unsigned m2l[W][TW_LIST];   // accepted nodes far from the group: into the group's local expansion
-  unsigned p2p[W][TW_LIST];   // near leaves: pairwise gravity + neighbour predicate
-  unsigned p2f[W][TW_LIST];   // far leaves: pairwise gravity only
-  unsigned hl[W][TW_LIST];    // far leaves queued for the classification of their halves
-  float4 src[W][32];   // staged sources: x, y, z, m
-  float4 q0[W][32];    // staged quadrupoles
-  float2 q1[W][32];
-  float2 sh[W][32];    // staged source index (bits) and smoothing length (direct list)
+  // A round of nodes leaves at most as many entries on the stack as it popped for each level below it: 32 F, and
+  // above HIGH only SLOW, so that the stack lasts for 48 levels of a tree opened throughout (56 with F = 4).
+  static constexpr int STACK = F == 1 ? 768 : 2560, HIGH = F == 1 ? 512 : 1280, SLOW = F == 1 ? 8 : 32;
+  static constexpr int LIST = F == 1 ? 96 : 256 * F;
+  static constexpr int FAR = F == 1 ? 448 : 256 * F;  // (long: a flush costs 31 shuffles)
+  static constexpr int SHORT = F == 1 ? 64 : 128 * F;
+  unsigned stack[STACK];
+  unsigned m2p[LIST];
+  unsigned m2l[FAR];     // accepted nodes far from the group: into the group's local expansion
+  unsigned p2f[LIST];    // far leaves: pairwise gravity only
+  unsigned p2p[SHORT];   // near leaves: pairwise gravity + neighbour predicate
+  unsigned hl[SHORT];    // far leaves queued for the classification of their halves
+  float4 src[F][32];     // staged sources: x, y, z, m; at the end the warps' sums of each particle
+  float4 q0[F][32];      // staged quadrupoles
+  float2 q1[F][32];
+  int idx[F][32];        // staged source indices and smoothing lengths (near leaves)
+  float hs[F][32];       // ... and the warps' sums of each coefficient of the local expansion
+  unsigned hits[2][F][F == 1 ? 1 : 32];  // neighbours each particle found in each warp's chunk (two rounds)
+  uint2 added[F];        // entries each warp adds in a round (two words of three counts)
+  unsigned stat[8];
 };
 
 // Compensated accumulator for the precision mode.
@@ -94,28 +120,28 @@ __device__ __forceinline__ void local_coeffs(float4 c, float4 q0, float2 q1, flo
   const float ex = ux * iR, ey = uy * iR, ez = uz * iR;
   const float s0 = G * c.w * iR, s1 = s0 * iR, s2 = s1 * iR, s3 = s2 * iR;
   const float xx = ex * ex, yy = ey * ey, zz2 = ez * ez;
-  v[0] = -s0;
-  v[1] = -s1 * ex;
-  v[2] = -s1 * ey;
-  v[3] = -s1 * ez;
-  v[4] = -s2 * fmaf(3.0f, xx, -1.0f);
-  v[5] = -s2 * fmaf(3.0f, yy, -1.0f);
-  v[6] = -s2 * fmaf(3.0f, zz2, -1.0f);
+  v[0] += -s0;
+  v[1] += -s1 * ex;
+  v[2] += -s1 * ey;
+  v[3] += -s1 * ez;
+  v[4] += -s2 * fmaf(3.0f, xx, -1.0f);
+  v[5] += -s2 * fmaf(3.0f, yy, -1.0f);
+  v[6] += -s2 * fmaf(3.0f, zz2, -1.0f);
   const float m3s2 = -3.0f * s2;
-  v[7] = m3s2 * ex * ey;
-  v[8] = m3s2 * ex * ez;
-  v[9] = m3s2 * ey * ez;
+  v[7] += m3s2 * ex * ey;
+  v[8] += m3s2 * ex * ez;
+  v[9] += m3s2 * ey * ez;
   const float ax = fmaf(-15.0f, xx, 3.0f), ay = fmaf(-15.0f, yy, 3.0f), az = fmaf(-15.0f, zz2, 3.0f);
-  v[10] = s3 * ex * (ax + 6.0f);
-  v[11] = s3 * ey * (ay + 6.0f);
-  v[12] = s3 * ez * (az + 6.0f);
-  v[13] = s3 * ey * ax;  // xxy
-  v[14] = s3 * ez * ax;  // xxz
-  v[15] = s3 * ex * ay;  // xyy
-  v[16] = s3 * ez * ay;  // yyz
-  v[17] = s3 * ex * az;  // xzz
-  v[18] = s3 * ey * az;  // yzz
-  v[19] = -15.0f * s3 * ex * ey * ez;
+  v[10] += s3 * ex * (ax + 6.0f);
+  v[11] += s3 * ey * (ay + 6.0f);
+  v[12] += s3 * ez * (az + 6.0f);
+  v[13] += s3 * ey * ax;  // xxy
+  v[14] += s3 * ez * ax;  // xxz
+  v[15] += s3 * ex * ay;  // xyy
+  v[16] += s3 * ez * ay;  // yyz
+  v[17] += s3 * ex * az;  // xzz
+  v[18] += s3 * ey * az;  // yzz
+  v[19] += -15.0f * s3 * ex * ey * ez;
   if (QUAD) {
     // q = G·Q (traceless, about the COM): φ = −½ eQe/R³; g = (Qe − 5/2 eQe e)/R⁴;
     // H = −(Q − 5(Qe eᵀ + e Qeᵀ) − 5/2 eQe I + 35/2 eQe e eᵀ)/R⁵
@@ -180,13 +206,35 @@ __device__ __forceinline__ void local_eval(const float cf[kLocal], float yx, flo
   }
 }
 
+// A particle meets itself in its own leaf: with soft2 above this, G m / soft2^1.5 stays finite for every G m below 3e20.
+constexpr float kNearSoft2 = 1.0e-12f;
+
 // What a gravity walk writes: the acceleration alone (a step's walk: the KDK integrator needs no potential),
 // the acceleration and the potential φ, or φ alone (into .w of the gravity record, for the energy diagnostic
 // of a state whose step walk left it out).
 enum { kWalkAcc = 0, kWalkAccPhi = 1, kWalkPhi = 2 };
 
-template <int W, bool GRAV, bool QUAD, bool NBR, bool HILO, int OUT>
-__global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
+// Minimum and maximum over the warp in one instruction (sm_100).
+__device__ __forceinline__ float warp_fmin(float v) {
+  float r;
+  asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float warp_fmax(float v) {
+  float r;
+  asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
+// The warps of a group meet (a warp of its own only orders its lanes).
+template <int F>
+__device__ __forceinline__ void group_sync() {
+  if constexpr (F == 1) __syncwarp();
+  else __syncthreads();
+}
+
+template <int F, bool GRAV, bool QUAD, bool NBR, bool HILO, int OUT>
+__global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
     const float4* __restrict__ body, const float4* __restrict__ pos_h, const double* __restrict__ x64,
     const double* __restrict__ y64, const double* __restrict__ z64, int K, int L,
     const unsigned* __restrict__ leaf_start, const unsigned long long* __restrict__ leaf_codes,
@@ -194,18 +242,17 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
     const float4* __restrict__ ncom, const float4* __restrict__ nbmin, const float4* __restrict__ nbmax, const float4* __restrict__ nq0,
     const float4* __restrict__ nq1, DevParams* P, float4* __restrict__ gout, unsigned* __restrict__ nbr,
     unsigned* __restrict__ nbr_cnt, unsigned cap, float skin, float* __restrict__ h0,
-    const uint2* __restrict__ groups, int ngroups, int stack_cap, float local_theta,
+    const uint2* __restrict__ groups, int stack_cap, float local_theta,
     int half, const float4* __restrict__ hcom, const float4* __restrict__ hq0, const float2* __restrict__ hq1,
     const float2* __restrict__ hrc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  WalkSmem<W>& S = *reinterpret_cast<WalkSmem<W>*>(smem_raw);
+  typedef WalkSmem<F> Smem;
+  Smem& S = *reinterpret_cast<Smem*>(smem_raw);
   const int w = threadIdx.x >> 5;
   const unsigned lane = threadIdx.x & 31u;
-  const int warp = blockIdx.x * W + w;
-  if (warp >= ngroups) return;
-  // this warp's group: a run of <= 32 Morton-consecutive particles of one impact (leaves g.x..g.y); the walk
-  // starts at that impact's root
-  const uint2 grp = groups[warp];
+  // this block's group: a run of <= 32 Morton-consecutive particles of one impact (leaves g.x..g.y), lane l of every
+  // warp holding particle l; the walk starts at that impact's root
+  const uint2 grp = groups[blockIdx.x];
   const int s0 = (int)leaf_start[grp.x], s1 = (int)leaf_start[grp.y + 1];
   const Seg& sgr = segs[(unsigned)(leaf_codes[grp.x] >> 30)];
   const unsigned root = sgr.root;
@@ -219,7 +266,7 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
     ylo = (float)(y64[t] - (double)pi.y);
     zlo = (float)(z64[t] - (double)pi.z);
   }
-  if (NBR && in_group && h0) h0[t] = pi.w;
+  if (NBR && in_group && h0 && w == 0) h0[t] = pi.w;
   // Split the group where consecutive particles are far apart (a leaf bucket of K consecutive Morton
   // particles can straddle a jump of the curve, e.g. between two bodies): each part walks with its own
   // compact box, so one straddling bucket cannot turn the walk into an all-pairs sum. The cut is at gaps above
@@ -253,28 +300,28 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
   // the packed sums of the far, near and multipole loops (two sources per FP32x2 instruction: half x for the
   // first source of each pair, half y for the second), folded into acc at the end
   float2 fx2 = make_float2(0.f, 0.f), fy2 = fx2, fz2 = fx2, fphi2 = fx2;
-  unsigned cnt = 0;
+  unsigned cnt = 0;       // neighbours of the lane's particle so far (the same in every warp)
   unsigned overflow = 0;
-  unsigned* stack = S.stack[w];
-  // per-warp counters, 32-bit (a warp's totals stay far below 2^32); the device totals are 64-bit
+  // this warp's counters, 32-bit (a block's totals stay far below 2^32); the device totals are 64-bit
   unsigned st_visits = 0, st_pops = 0, st_m2p = 0, st_p2p = 0, st_m2l = 0, st_slots = 0;
+  if (threadIdx.x < 8) S.stat[threadIdx.x] = 0u;
 
   for (int part = 0; part < nparts; ++part) {
   const bool valid = in_group && mypart == part;
   const float big = 3.0e38f;
-  const float gx0 = warp_min(valid ? pi.x : big), gy0 = warp_min(valid ? pi.y : big),
-              gz0 = warp_min(valid ? pi.z : big);
-  const float gx1 = warp_max(valid ? pi.x : -big), gy1 = warp_max(valid ? pi.y : -big),
-              gz1 = warp_max(valid ? pi.z : -big);
-  const float ghmax = warp_max(valid ? pi.w : 0.0f);
+  const float gx0 = warp_fmin(valid ? pi.x : big), gy0 = warp_fmin(valid ? pi.y : big),
+              gz0 = warp_fmin(valid ? pi.z : big);
+  const float gx1 = warp_fmax(valid ? pi.x : -big), gy1 = warp_fmax(valid ? pi.y : -big),
+              gz1 = warp_fmax(valid ? pi.z : -big);
+  const float ghmax = warp_fmax(valid ? pi.w : 0.0f);
   // the part's local expansion: centre z, and the distance beyond which an accepted node's COM joins it
   const float zx = 0.5f * (gx0 + gx1), zy = 0.5f * (gy0 + gy1), zz = 0.5f * (gz0 + gz1);
   const float rg2 = 0.25f * ((gx1 - gx0) * (gx1 - gx0) + (gy1 - gy0) * (gy1 - gy0) + (gz1 - gz0) * (gz1 - gz0));
   const float far2 = (GRAV && local_theta > 0.0f) ? rg2 / (local_theta * local_theta) : big;
-  float loc = 0.0f;  // lane k < kLocal: coefficient k of the part's expansion
+  float loc = 0.0f;  // lane k < kLocal: this warp's sum of coefficient k of the part's expansion
   int sp = 1, nm = 0, np = 0, nf = 0, nl = 0;
-  if (lane == 0) stack[0] = root;
-  __syncwarp();
+  if (threadIdx.x == 0) S.stack[0] = root;
+  group_sync<F>();
 
   // ---- far leaves: branch-free pairwise gravity, 32 staged sources per pass ---------------------------
   // The next chunk's sources are loaded into registers before this chunk is evaluated, so the gather
@@ -287,7 +334,7 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
     float4 src = make_float4(3.0e18f, 3.0e18f, 3.0e18f, 0.0f);  // padding: massless and far away
     real = false;
     if (li < min(per, count - base)) {
-      const unsigned e = S.p2f[w][base + li];  // first source << 5 | (sources − 1)
+      const unsigned e = S.p2f[base + li];  // first source << 5 | (sources − 1)
       if (off <= (int)(e & 31u)) {
         src = body[(e >> 5) + off];
         real = true;
@@ -299,12 +346,16 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
   // consecutive float4, and each pair is evaluated with the packed FP32x2 operations of sm_100 (add, multiply
   // and fused multiply-add on two lanes of a register pair, each rounded as its scalar form): one instruction
   // does both sources' arithmetic, the reciprocal square roots stay scalar.
-  auto flush_far = [&](int count) {
+  auto flush_far = [&](int total) {
     const int per = far_per;
-    part_p2p += (unsigned)count << kfsh;
+    // this warp's share of the list, in whole chunks
+    const int share = F == 1 ? total : ((total + per - 1) / per + F - 1) / F * per;
+    const int first = w * share, count = min(total, first + share);
+    if (first >= count) return;
+    part_p2p += (unsigned)(count - first) << kfsh;
     bool nreal;
-    float4 nxt = far_source(0, count, nreal);
-    for (int base = 0; base < count; base += per) {
+    float4 nxt = far_source(first, count, nreal);
+    for (int base = first; base < count; base += per) {
       float4 src = nxt;
       part_src += __popc(__ballot_sync(SPH_FULL_MASK, nreal));
       if (base + per < count) nxt = far_source(base + per, count, nreal);
@@ -377,35 +428,36 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
     }
   };
 
-  // ---- far multipoles: each lane expands its own node about z, the warp sums the coefficients -------------
-  auto flush_m2l = [&](int count) {
-    for (int base = 0; base < count; base += 32) {
-      float v[32];
+  // ---- far multipoles: each lane expands its own nodes about z and keeps the sums of their coefficients; the warp
+  // sums them once, at the end of its share ------------------------------------------------------------------
+  auto flush_m2l = [&](int total) {
+    float v[32];
 #pragma unroll
-      for (int k = 0; k < 32; ++k) v[k] = 0.0f;
-      if ((int)lane < count - base) {
-        float4 c, q0;
-        float2 q1;
-        load_multipole(S.m2l[w][base + lane], c, q0, q1);
-        local_coeffs<QUAD>(c, q0, q1, G, zx, zy, zz, soft2, v);
-      }
-      loc += warp_transpose_sum32(v);
+    for (int k = 0; k < 32; ++k) v[k] = 0.0f;
+    for (int i = (int)threadIdx.x; i < total; i += F * 32) {
+      float4 c, q0;
+      float2 q1;
+      load_multipole(S.m2l[i], c, q0, q1);
+      local_coeffs<QUAD>(c, q0, q1, G, zx, zy, zz, soft2, v);
     }
+    loc += warp_transpose_sum32(v);
   };
 
   // ---- multipole list: stage 32 nodes in shared memory, then every lane applies them -------------------
   // Without hi/lo coordinates the nodes are staged in pairs, (x₀ x₁ y₀ y₁)(z₀ z₁ m₀ m₁) in src,
   // (Qxx Qyy)(Qzz Qxy) pairs in q0 and (Qxz Qyz) pairs in q1, and evaluated two at a time with the packed
   // FP32x2 operations; an odd chunk is padded with a massless node far away.
-  auto flush_m2p = [&](int count) {
-    for (int base = 0; base < count; base += 32) {
+  auto flush_m2p = [&](int total) {
+    const int share = F == 1 ? total : ((total + 2 * F - 1) / (2 * F)) * 2;  // this warp's share of the list, in pairs
+    const int first = w * share, count = min(total, first + share);
+    for (int base = first; base < count; base += 32) {
       const int m = min(32, count - base);
       if (HILO) {
         if ((int)lane < m) {
           // staged with G folded in: (com, G·M) and G·Q
           float4 c, q;
           float2 b;
-          load_multipole(S.m2p[w][base + lane], c, q, b);
+          load_multipole(S.m2p[base + lane], c, q, b);
           c.w *= G;
           S.src[w][lane] = c;
           if (QUAD) {
@@ -416,7 +468,7 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
       } else if ((int)lane < ((m + 1) & ~1)) {
         float4 c = make_float4(3.0e18f, 3.0e18f, 3.0e18f, 0.0f), q = make_float4(0.f, 0.f, 0.f, 0.f);
         float2 b = make_float2(0.f, 0.f);
-        if ((int)lane < m) load_multipole(S.m2p[w][base + lane], c, q, b);
+        if ((int)lane < m) load_multipole(S.m2p[base + lane], c, q, b);
         float* f = reinterpret_cast<float*>(&S.src[w][0]) + 8 * (lane >> 1) + (lane & 1u);
         f[0] = c.x;
         f[2] = c.y;
@@ -524,7 +576,7 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
     const int per = near_per, li = near_li, off = near_off;  // leaves per chunk, this lane's leaf and source
     int sidx = -1;
     if (li < min(per, count - base)) {
-      const unsigned e = S.p2p[w][base + li];  // first source << 5 | (sources − 1)
+      const unsigned e = S.p2p[base + li];  // first source << 5 | (sources − 1)
       if (off <= (int)(e & 31u)) sidx = (int)(e >> 5) + off;
     }
     src = make_float4(3.0e18f, 3.0e18f, 3.0e18f, 0.0f);  // padding: massless and far away
@@ -535,27 +587,20 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
     }
     return sidx;
   };
-  // The neighbour test and the append of one source that passed it (the list keeps the chunk's order).
+  // The sources of a chunk that passed the neighbour test, one bit each (the first source's bit highest).
+  unsigned found = 0u;
   // (the particle's first list slot once, entries 32 apart: the interleaved layout of nbr_slot)
   unsigned* const nlst = NBR ? nbr + nbr_slot((unsigned)t, 0u, cap) : nullptr;
-  auto near_append = [&](bool inside, int s) {
-    if (inside) {
-      if (cnt < cap) nlst[(size_t)cnt * 32u] = (unsigned)s;
-      ++cnt;
-    }
-  };
-  // Without hi/lo coordinates: sources in pairs, as in the far loop (the pair (x₀ x₁ y₀ y₁)(z₀ z₁ m₀ m₁) and
-  // (index₀ index₁ h₀ h₁)); every packed operation rounds as its scalar form, so the distances and the
-  // predicate are those of the scalar loop below, source by source.
+  // Sources in pairs, as in the far loop (their smoothing lengths in hs); every packed operation rounds as its scalar
+  // form, so the distances and the predicate are those of the scalar loop below, source by source. A test is the sign
+  // of d² − lim², shifted into `found`. The particle itself goes through the loop like any other source: at d = 0 its
+  // force is a finite number times zero (soft2 >= kNearSoft2), flush_p2p takes its bit and its potential back.
   auto near_pairs = [&](auto loose) {
     const float2 npx = make_float2(-pi.x, -pi.x), npy = make_float2(-pi.y, -pi.y), npz = make_float2(-pi.z, -pi.z);
     const float2 s2 = make_float2(soft2, soft2);
-    const float4* shp = reinterpret_cast<const float4*>(&S.sh[w][0]);
 #pragma unroll 2
     for (int k = 0; k < 16; ++k) {
-      const float4 xy = S.src[w][2 * k], zm = S.src[w][2 * k + 1], sh = shp[k];
-      const int sa = __float_as_int(sh.x), sb = __float_as_int(sh.y);
-      const bool oa = sa != t, ob = sb != t;
+      const float4 xy = S.src[w][2 * k], zm = S.src[w][2 * k + 1];
       const float2 dx = __fadd2_rn(make_float2(xy.x, xy.y), npx);
       const float2 dy = __fadd2_rn(make_float2(xy.z, xy.w), npy);
       const float2 dz = __fadd2_rn(make_float2(zm.x, zm.y), npz);
@@ -563,65 +608,60 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
       if constexpr (decltype(loose)::value) dd = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
       else dd = __fadd2_rn(__fadd2_rn(__fmul2_rn(dx, dx), __fmul2_rn(dy, dy)), __fmul2_rn(dz, dz));
       if (NBR) {
-        bool ia, ib;
+        const float2 h = *reinterpret_cast<const float2*>(&S.hs[w][2 * k]);
         if constexpr (decltype(loose)::value) {
-          const float2 lim = __ffma2_rn(make_float2(sh.z, sh.w), make_float2(lim_j, lim_j), make_float2(lim_i, lim_i));
-          const float2 l2 = __fmul2_rn(lim, lim);
-          ia = dd.x < l2.x;
-          ib = dd.y < l2.y;
+          const float2 lim = __ffma2_rn(h, make_float2(lim_j, lim_j), make_float2(lim_i, lim_i));
+          const float2 in = __ffma2_rn(make_float2(-lim.x, -lim.y), lim, dd);  // negative inside
+          found = __funnelshift_l(__float_as_uint(in.x), found, 1);
+          found = __funnelshift_l(__float_as_uint(in.y), found, 1);
         } else {
-          const float2 lim = __fmul2_rn(make_float2(0.5f, 0.5f), __fadd2_rn(make_float2(pi.w, pi.w), make_float2(sh.z, sh.w)));
+          const float2 lim = __fmul2_rn(make_float2(0.5f, 0.5f), __fadd2_rn(make_float2(pi.w, pi.w), h));
           const float2 q = __fmul2_rn(lim, lim);
           const float2 qlo = __fmul2_rn(q, make_float2(1.0f - 1.9073486e-6f, 1.0f - 1.9073486e-6f));
           const float2 qhi = __fmul2_rn(q, make_float2(1.0f + 1.9073486e-6f, 1.0f + 1.9073486e-6f));
-          ia = dd.x < qlo.x;
+          bool ia = dd.x < qlo.x, ib = dd.y < qlo.y;
           if (!ia && !(dd.x > qhi.x)) ia = fsqrt(dd.x) < lim.x;
-          ib = dd.y < qlo.y;
           if (!ib && !(dd.y > qhi.y)) ib = fsqrt(dd.y) < lim.y;
+          found = found << 2 | (ia ? 2u : 0u) | (ib ? 1u : 0u);
         }
-        near_append(oa && ia, sa);
-        near_append(ob && ib, sb);
       }
       if (GRAV) {
-        // the particle itself (d = 0) gets r² = 1: a finite g times a zero offset adds nothing
-        const float2 r2s = __fadd2_rn(dd, s2);
-        const float2 r2 = make_float2(oa ? r2s.x : 1.0f, ob ? r2s.y : 1.0f);
+        const float2 r2 = __fadd2_rn(dd, s2);
         const float2 rinv = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
         const float2 gm = __fmul2_rn(make_float2(zm.z, zm.w), rinv);
         const float2 g = __fmul2_rn(__fmul2_rn(gm, rinv), rinv);
         fx2 = __ffma2_rn(g, dx, fx2);
         fy2 = __ffma2_rn(g, dy, fy2);
         fz2 = __ffma2_rn(g, dz, fz2);
-        if (OUT != kWalkAcc) fphi2 = __fadd2_rn(fphi2, make_float2(oa ? -gm.x : 0.0f, ob ? -gm.y : 0.0f));
+        if (OUT != kWalkAcc) fphi2 = __fadd2_rn(fphi2, make_float2(-gm.x, -gm.y));
       }
     }
   };
+  // One source at a time: hi/lo coordinates, and softenings too small for the particle's own term above.
   auto near_sources = [&](auto loose) {
 #pragma unroll 4
     for (int k = 0; k < 32; ++k) {
-      const float2 shk = S.sh[w][k];
-      const int s = __float_as_int(shk.x);
-      // padding (s = −1) sits massless at 3e18: it passes no neighbour test and adds no gravity
-      const bool other = s != t;
+      // padding (index −1) sits massless at 3e18: it passes no neighbour test and adds no gravity
+      const bool other = S.idx[w][k] != t;
       const float4 bj = S.src[w][k];
       const float dx = fsub(bj.x, pi.x), dy = fsub(bj.y, pi.y), dz = fsub(bj.z, pi.z);
       // the exact predicate needs the single-rounded distance; the conservative one's 2^-19 margin is far above
       // the few ulp a fused form differs by
       const float dd = decltype(loose)::value ? fmaf(dz, dz, fmaf(dy, dy, dx * dx)) : dot3_exact(dx, dy, dz);
-      if (NBR && other) {
+      if (NBR) {
         bool inside;
         if constexpr (decltype(loose)::value) {
-          const float lim = fmaf(shk.y, lim_j, lim_i);
+          const float lim = fmaf(S.hs[w][k], lim_j, lim_i);
           inside = dd < lim * lim;
         } else {
-          const float lim = fmul(0.5f, fadd(pi.w, shk.y));
+          const float lim = fmul(0.5f, fadd(pi.w, S.hs[w][k]));
           // sqrt_rn(dd) < lim, decided without the square root outside a 2^-19 band around lim²:
           // dd < lim²(1-2^-19) ⇒ √dd < lim − 2 ulp(lim); dd > lim²(1+2^-19) ⇒ √dd > lim + 2 ulp(lim)
           const float q = fmul(lim, lim);
           inside = dd < fmul(q, 1.0f - 1.9073486e-6f);
           if (!inside && !(dd > fmul(q, 1.0f + 1.9073486e-6f))) inside = fsqrt(dd) < lim;
         }
-        near_append(inside, s);
+        found = found << 1 | (inside ? 1u : 0u);
       }
       if (GRAV) {
         float ex = dx, ey = dy, ez = dz, d2 = dd;
@@ -642,60 +682,100 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
       }
     }
   };
+  // Rounds of F chunks, one for each warp; a particle's list takes the warps' finds in their order, so the list is
+  // that of a single warp going through the chunks.
+  const bool one_by_one = HILO || (GRAV && soft2 < kNearSoft2);
   auto flush_p2p = [&](int count) {
     const int per = near_per;  // leaves per chunk
     float4 nsrc;
     float nh;
-    part_p2p += (unsigned)count << ksh;
-    int nidx = near_source(0, count, nsrc, nh);
-    for (int base = 0; base < count; base += per) {
+    int nidx = near_source(w * per, count, nsrc, nh);
+    unsigned turn = 0u;
+    for (int base = 0; base < count; base += per * F, turn ^= 1u) {
+      const int mine = base + w * per;
       float4 src = nsrc;
       const float hsrc = nh;
       const int sidx = nidx;
-      part_src += __popc(__ballot_sync(SPH_FULL_MASK, sidx >= 0));
-      if (base + per < count) nidx = near_source(base + per, count, nsrc, nh);
-      src.w *= G;
-      if (HILO) {
-        S.src[w][lane] = src;
-        S.sh[w][lane] = make_float2(__int_as_float(sidx), hsrc);
-      } else {
-        float* f = reinterpret_cast<float*>(&S.src[w][0]) + 8 * (lane >> 1) + (lane & 1u);
-        f[0] = src.x;
-        f[2] = src.y;
-        f[4] = src.z;
-        f[6] = src.w;
-        float* e = reinterpret_cast<float*>(&S.sh[w][0]) + 4 * (lane >> 1) + (lane & 1u);
-        e[0] = __int_as_float(sidx);
-        e[2] = hsrc;
+      found = 0u;
+      if (mine < count) {  // (the warp)
+        part_p2p += (unsigned)min(per, count - mine) << ksh;
+        part_src += __popc(__ballot_sync(SPH_FULL_MASK, sidx >= 0));
+        nidx = near_source(mine + per * F, count, nsrc, nh);
+        src.w *= G;
+        S.idx[w][lane] = sidx;
+        if (NBR) S.hs[w][lane] = hsrc;
+        if (one_by_one) {
+          S.src[w][lane] = src;
+        } else {
+          float* f = reinterpret_cast<float*>(&S.src[w][0]) + 8 * (lane >> 1) + (lane & 1u);
+          f[0] = src.x;
+          f[2] = src.y;
+          f[4] = src.z;
+          f[6] = src.w;
+        }
+        // the place of each of the group's particles among this chunk's sources, if the chunk holds any of them
+        const bool own = sidx >= s0 && sidx < s1;
+        const bool holds_own = __any_sync(SPH_FULL_MASK, own);
+        int* place = reinterpret_cast<int*>(&S.q1[w][0]);
+        if (holds_own) {
+          place[lane] = 32;
+          __syncwarp();
+          if (own) place[sidx - s0] = (int)lane;
+        }
+        __syncwarp();
+        if (valid) {
+          // A list built with a skin is a candidate set: the gather kernels keep r < h_ij at the current h,
+          // and the smoothing-length solve holds h below h0·(1 + skin)·0.999, so every superset of the exact
+          // predicate gives the same sums in the same order. With a skin the test is therefore a conservative
+          // one (lim padded by 2^-19, more than the rounding of either form); without one (fixed h) it is the
+          // reference's exact predicate.
+          if (one_by_one) {
+            if (NBR && skin > 0.0f) near_sources(std::true_type{});
+            else near_sources(std::false_type{});
+          } else {
+            if (NBR && skin > 0.0f) near_pairs(std::true_type{});
+            else near_pairs(std::false_type{});
+          }
+          if (holds_own && place[lane] < 32) {
+            found &= ~(0x80000000u >> place[lane]);
+            if (GRAV && OUT != kWalkAcc && !one_by_one) phi += fmul(fmul(body[t].w, G), rsqrt_ftz(soft2));
+          }
+        }
       }
-      __syncwarp();
-      if (valid && !HILO) {
-        if (NBR && skin > 0.0f) near_pairs(std::true_type{});
-        else near_pairs(std::false_type{});
-      }
-      if (valid && HILO) {
-        // A list built with a skin is a candidate set: the gather kernels keep r < h_ij at the current h,
-        // and the smoothing-length solve holds h below h0·(1 + skin)·0.999, so every superset of the exact
-        // predicate gives the same sums in the same order. With a skin the test is therefore a conservative
-        // one (lim padded by 2^-19, more than the rounding of either form); without one (fixed h) it is the
-        // reference's exact predicate.
-        if (NBR && skin > 0.0f) near_sources(std::true_type{});
-        else near_sources(std::false_type{});
+      if (NBR) {
+        unsigned at = cnt;
+        if constexpr (F == 1) {
+          cnt += (unsigned)__popc(found);
+        } else {
+          S.hits[turn][w][lane] = (unsigned)__popc(found);
+          __syncthreads();
+#pragma unroll
+          for (int k = 0; k < F; ++k) {
+            const unsigned h = S.hits[turn][k][lane];
+            at += k < w ? h : 0u;
+            cnt += h;
+          }
+        }
+        for (; found; ++at) {
+          const int k = __clz(found);
+          found &= ~(0x80000000u >> k);
+          if (at < cap) nlst[(size_t)at * 32u] = (unsigned)S.idx[w][k];
+        }
       }
       __syncwarp();
     }
   };
 
   const unsigned nvalid = __popc(__ballot_sync(SPH_FULL_MASK, valid));
-  // One pass per pop; the pass after the stack empties flushes what the lists still hold, so that every flush
-  // loop has one call site (the walk's hot code is instruction-cache bound: a second inlined copy of each flush
-  // loop measurably stalled instruction fetch). With half leaves a pass is of one of two kinds: a pop of up to
-  // 32 nodes, whose far leaves are queued (S.hl), or a batch of up to 32 queued far leaves whose halves are
-  // classified, one leaf per lane. Classifying halves in the pop that found the leaf ran that code once per pop
-  // with a few lanes active; batched, it runs once per 32 leaves.
+  // The warps take the rounds together, 32 entries to each warp, and list what they find in the warps' order. The round
+  // after the stack empties flushes what the lists still hold, so that every flush loop has one call site (the walk's
+  // hot code is instruction-cache bound: a second inlined copy of each flush loop measurably stalled instruction
+  // fetch). With half leaves a round is of one of two kinds: a pop of nodes, whose far leaves are queued (S.hl), or a
+  // batch of queued far leaves whose halves are classified, one leaf per lane (in the pop that found the leaf that code
+  // ran with a few lanes active).
   int nq = 0;  // far leaves queued for the half classification
   for (;;) {
-  const bool halves = GRAV && half > 0 && (nq >= 32 || (sp == 0 && nq > 0));
+  const bool halves = GRAV && half > 0 && (nq >= 32 * F || (sp == 0 && nq > 0));
   const bool done = sp == 0 && nq == 0;
   if (!done) {
     // Entries of this lane: a node for the multipole lists (m0 per particle, l0 into the group's expansion), a
@@ -709,12 +789,16 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
     unsigned ls0 = 0u, ls1 = 1u;                    // a leaf's source range
     unsigned lc = 0u, rc = 0u;                      // an internal node's children, loaded alongside its box
     unsigned node = 0u;
+    // the nodes or queued leaves of this round, above sp or nq once taken
+    const int take = halves ? min(nq, 32 * F) : min(sp, sp > Smem::HIGH ? Smem::SLOW : 32 * F);
+    if (halves) nq -= take;
+    else sp -= take;
+    const bool have = (int)threadIdx.x < take;
+    unsigned bm0 = 0u, bm1 = 0u, bl0 = 0u, bl1 = 0u, bf0 = 0u, bf1 = 0u, bo = 0u, bn = 0u, bq = 0u;
+    if (F == 1 || 32 * w < take) {  // (the warp)
     if (halves) {
-      const int take = min(nq, 32);
-      nq -= take;
-      const bool have = (int)lane < take;
-      const unsigned cl = have ? S.hl[w][nq + (int)lane] : 0u;
-      __syncwarp();
+      const unsigned cl = have ? S.hl[nq + (int)threadIdx.x] : 0u;
+      if (F == 1) __syncwarp();
       if (have) {
         ls0 = leaf_start[cl];
         ls1 = leaf_start[cl + 1];
@@ -750,13 +834,10 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
         }
       }
     } else {
-      const int take = min(sp, 32);
-      sp -= take;
-      st_visits += take;
+      node = have ? S.stack[sp + threadIdx.x] : 0u;
+      if (F == 1) __syncwarp();
+      st_visits += min(32, take - 32 * w);
       ++st_pops;
-      const bool have = (int)lane < take;
-      node = have ? stack[sp + lane] : 0u;
-      __syncwarp();
       bool acc_node = false, leaf = false, far_l = false;
       float4 lbl = make_float4(0.f, 0.f, 0.f, 0.f), lbh = lbl;  // the node's box (and max h), for the lane test
       if (have) {
@@ -799,11 +880,12 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
         if (is_leaf && ls1 <= ls0) acc_node = leaf = false;  // an empty leaf (none are built) adds nothing
         near_leaf = leaf && near;
       }
-      if (NBR && GRAV) {
+      if (NBR && GRAV && half > 0) {
         // A leaf near the group box may still be out of every particle's own reach: then it can hold no
         // neighbour and takes the cheaper far path. The test is conservative (reach with the list's skin and a
         // margin), and a leaf holding a particle of the part is at distance 0, so self-pairs stay on the near
-        // path.
+        // path. It pays for leaves of 16 and more, whose far halves may become multipoles; for smaller ones, summed
+        // pairwise on either path, it cost more than it saved (219 against 148 µs at 10,240 particles in leaves of 1).
         const unsigned cand = __ballot_sync(SPH_FULL_MASK, near_leaf);
         unsigned keep = 0;
         for (unsigned b = cand; b; b &= b - 1) {
@@ -828,95 +910,152 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
       f0 = far_leaf && !queue;
       fe0 = (ls0 << 5) | min(ls1 - ls0 - 1u, 31u);
     }
-    const unsigned bm0 = __ballot_sync(SPH_FULL_MASK, m0), bm1 = __ballot_sync(SPH_FULL_MASK, m1);
-    const unsigned bl0 = __ballot_sync(SPH_FULL_MASK, l0), bl1 = __ballot_sync(SPH_FULL_MASK, l1);
-    const unsigned bf0 = __ballot_sync(SPH_FULL_MASK, f0), bf1 = __ballot_sync(SPH_FULL_MASK, f1);
-    const unsigned bo = __ballot_sync(SPH_FULL_MASK, open);
-    const unsigned bn = __ballot_sync(SPH_FULL_MASK, near_leaf);
-    const unsigned bq = __ballot_sync(SPH_FULL_MASK, queue);
-    if (queue) S.hl[w][nq + __popc(bq & lt)] = node - leaf0;
-    nq += __popc(bq);
+    bm0 = __ballot_sync(SPH_FULL_MASK, m0), bm1 = __ballot_sync(SPH_FULL_MASK, m1);
+    bl0 = __ballot_sync(SPH_FULL_MASK, l0), bl1 = __ballot_sync(SPH_FULL_MASK, l1);
+    bf0 = __ballot_sync(SPH_FULL_MASK, f0), bf1 = __ballot_sync(SPH_FULL_MASK, f1);
+    bo = __ballot_sync(SPH_FULL_MASK, open);
+    bn = __ballot_sync(SPH_FULL_MASK, near_leaf);
+    bq = __ballot_sync(SPH_FULL_MASK, queue);
+    }  // the warp
+    // the round's entries in the warps' order: each warp's counts, ten bits each, and their prefix
+    uint2 before = make_uint2(0u, 0u), all;
+    all.x = (unsigned)(__popc(bm0) + __popc(bm1)) | (unsigned)(__popc(bl0) + __popc(bl1)) << 10 |
+            (unsigned)(__popc(bf0) + __popc(bf1)) << 20;
+    all.y = (unsigned)__popc(bo) | (unsigned)__popc(bn) << 10 | (unsigned)__popc(bq) << 20;
+    if constexpr (F > 1) {
+      if (lane == 0) S.added[w] = all;
+      __syncthreads();  // ... and every warp has read its nodes
+      const uint2 a = S.added[lane & (F - 1)];
+      before.x = __reduce_add_sync(SPH_FULL_MASK, (int)lane < w ? a.x : 0u);
+      before.y = __reduce_add_sync(SPH_FULL_MASK, (int)lane < w ? a.y : 0u);
+      all.x = __reduce_add_sync(SPH_FULL_MASK, lane < (unsigned)F ? a.x : 0u);
+      all.y = __reduce_add_sync(SPH_FULL_MASK, lane < (unsigned)F ? a.y : 0u);
+    }
+    if (queue) S.hl[nq + (int)(before.y >> 20) + __popc(bq & lt)] = node - leaf0;
     // two entries per lane: lanes below this one come first, then this lane's first and second entry
     if (m0 || m1) {
-      const int k = nm + __popc(bm0 & lt) + __popc(bm1 & lt);
-      if (m0) S.m2p[w][k] = v0;
-      if (m1) S.m2p[w][k + (m0 ? 1 : 0)] = v1;
+      const int k = nm + (int)(before.x & 1023u) + __popc(bm0 & lt) + __popc(bm1 & lt);
+      if (m0) S.m2p[k] = v0;
+      if (m1) S.m2p[k + (m0 ? 1 : 0)] = v1;
     }
     if (l0 || l1) {
-      const int k = nl + __popc(bl0 & lt) + __popc(bl1 & lt);
-      if (l0) S.m2l[w][k] = v0;
-      if (l1) S.m2l[w][k + (l0 ? 1 : 0)] = v1;
+      const int k = nl + (int)(before.x >> 10 & 1023u) + __popc(bl0 & lt) + __popc(bl1 & lt);
+      if (l0) S.m2l[k] = v0;
+      if (l1) S.m2l[k + (l0 ? 1 : 0)] = v1;
     }
     if (f0 || f1) {
-      const int k = nf + __popc(bf0 & lt) + __popc(bf1 & lt);
-      if (f0) S.p2f[w][k] = fe0;
-      if (f1) S.p2f[w][k + (f0 ? 1 : 0)] = fe1;
+      const int k = nf + (int)(before.x >> 20) + __popc(bf0 & lt) + __popc(bf1 & lt);
+      if (f0) S.p2f[k] = fe0;
+      if (f1) S.p2f[k + (f0 ? 1 : 0)] = fe1;
     }
     // list entries carry the leaf's source range (capacity <= 2^26 particles, leaves <= 32 sources)
-    if (near_leaf) S.p2p[w][np + __popc(bn & lt)] = (ls0 << 5) | min(ls1 - ls0 - 1u, 31u);
-    const int no = __popc(bo);
+    if (near_leaf) S.p2p[np + (int)(before.y >> 10 & 1023u) + __popc(bn & lt)] = (ls0 << 5) | min(ls1 - ls0 - 1u, 31u);
+    const int no = (int)(all.y & 1023u);
     if (sp + 2 * no <= stack_cap) {
       if (open) {
-        const int r = sp + 2 * __popc(bo & lt);
-        stack[r] = lc;
-        stack[r + 1] = rc;
+        const int r = sp + 2 * ((int)(before.y & 1023u) + __popc(bo & lt));
+        S.stack[r] = lc;
+        S.stack[r + 1] = rc;
       }
       sp += 2 * no;
     } else if (no) {
       overflow = 1;
     }
-    nm += __popc(bm0) + __popc(bm1);
-    nl += __popc(bl0) + __popc(bl1);
-    np += __popc(bn);
-    nf += __popc(bf0) + __popc(bf1);
-    part_m2p += __popc(bm0) + __popc(bm1);
-    part_m2l += __popc(bl0) + __popc(bl1);
+    const int am = (int)(all.x & 1023u), al = (int)(all.x >> 10 & 1023u);
+    nm += am;
+    nl += al;
+    nf += (int)(all.x >> 20);
+    np += (int)(all.y >> 10 & 1023u);
+    nq += (int)(all.y >> 20);
+    part_m2p += am;
+    part_m2l += al;
   }  // !done
-    __syncwarp();
-    if (nm > TW_LIST - 64 || (done && nm)) {
+    group_sync<F>();
+    if (nm > Smem::LIST - 64 * F || (done && nm)) {
       flush_m2p(nm);
       nm = 0;
     }
-    if (nl > TW_LIST - 64 || (done && nl)) {
+    if (nl > Smem::FAR - 64 * F || (done && nl)) {
       flush_m2l(nl);
       nl = 0;
     }
-    if (np > TW_LIST - 64 || (done && np)) {
+    if (np > Smem::SHORT - 32 * F || (done && np)) {
       flush_p2p(np);
       np = 0;
     }
-    if (nf > TW_LIST - 64 || (done && nf)) {
+    if (nf > Smem::LIST - 64 * F || (done && nf)) {
       flush_far(nf);
       nf = 0;
     }
     if (done) break;
   }
   if (GRAV && part_m2l) {
-    // the part's expansion (lane k holds coefficient k) evaluated by every particle of the part
-    float cf[kLocal];
+    // the part's expansion (lane k holds coefficient k) evaluated by every particle of the part, in the first warp
+    if constexpr (F > 1) {
+      S.hs[w][lane] = loc;  // (the near sources' smoothing lengths are done with)
+      __syncthreads();
+    }
+    if (w == 0) {
 #pragma unroll
-    for (int k = 0; k < kLocal; ++k) cf[k] = __shfl_sync(SPH_FULL_MASK, loc, k);
-    if (valid) {
-      float yx = pi.x - zx, yy = pi.y - zy, yz = pi.z - zz;
-      if (HILO) { yx += xlo; yy += ylo; yz += zlo; }
-      float lx, ly, lz;
-      local_eval<OUT != kWalkAcc>(cf, yx, yy, yz, lx, ly, lz, phi);
-      acc.add<HILO>(lx, ly, lz);
+      for (int k = 1; k < F; ++k) loc += S.hs[k][lane];
+      float cf[kLocal];
+#pragma unroll
+      for (int k = 0; k < kLocal; ++k) cf[k] = __shfl_sync(SPH_FULL_MASK, loc, k);
+      if (valid) {
+        float yx = pi.x - zx, yy = pi.y - zy, yz = pi.z - zz;
+        if (HILO) { yx += xlo; yy += ylo; yz += zlo; }
+        float lx, ly, lz;
+        local_eval<OUT != kWalkAcc>(cf, yx, yy, yz, lx, ly, lz, phi);
+        acc.add<HILO>(lx, ly, lz);
+      }
     }
   }
   st_m2p += part_m2p * nvalid;                             // node × particle interactions
   st_m2l += part_m2l;                                      // nodes expanded about a part's centre
   st_p2p += part_src * nvalid;                             // source particles × particles
   st_slots += part_p2p * nvalid;                           // ... counting the slots the lanes ran
+  group_sync<F>();  // every warp is done with the lists before the next part's
   }  // parts
 
-  if (in_group && GRAV) {
+  if (GRAV) {
+    // the warps' sums in the warps' order
     if (!HILO) {
       acc.add<false>(fx2.x + fx2.y, fy2.x + fy2.y, fz2.x + fz2.y);
       phi += fphi2.x + fphi2.y;
+    } else {
+      acc.x -= acc.cx;
+      acc.y -= acc.cy;
+      acc.z -= acc.cz;
     }
-    if (OUT == kWalkPhi) reinterpret_cast<float*>(gout)[4 * (size_t)t + 3] = phi;
-    else gout[t] = make_float4(acc.x, acc.y, acc.z, OUT == kWalkAccPhi ? phi : 0.0f);
+    S.src[w][lane] = make_float4(acc.x, acc.y, acc.z, phi);
+  }
+  // the block's counters (a diagnostic's potential walk is not a step's walk): multipoles as every warp counted them
+  if (OUT != kWalkPhi && lane == 0) {
+    if constexpr (F == 1) {
+      S.stat[0] = st_visits, S.stat[1] = st_pops, S.stat[2] = st_m2p;
+      S.stat[3] = st_p2p, S.stat[4] = st_m2l, S.stat[5] = st_slots;
+    } else {
+      atomicAdd(&S.stat[0], st_visits);
+      atomicAdd(&S.stat[1], st_pops);
+      atomicAdd(&S.stat[3], st_p2p);
+      atomicAdd(&S.stat[5], st_slots);
+      if (w == 0) S.stat[2] = st_m2p, S.stat[4] = st_m2l;
+    }
+  }
+  group_sync<F>();
+  if (w != 0) return;
+  if (in_group && GRAV) {
+    float4 r = S.src[0][lane];
+#pragma unroll
+    for (int k = 1; k < F; ++k) {
+      const float4 v = S.src[k][lane];
+      r.x += v.x;
+      r.y += v.y;
+      r.z += v.z;
+      r.w += v.w;
+    }
+    if (OUT == kWalkPhi) reinterpret_cast<float*>(gout)[4 * (size_t)t + 3] = r.w;
+    else gout[t] = make_float4(r.x, r.y, r.z, OUT == kWalkAccPhi ? r.w : 0.0f);
   }
   if (NBR) {
     if (in_group) nbr_cnt[t] = cnt;
@@ -927,73 +1066,59 @@ __global__ void __launch_bounds__(W * 32, TW_WARPS_PER_SM / W) k_tree_walk(
     }
   }
   if (overflow && lane == 0) atomicOr(&P->flags, kFlagStackOverflow);
-  if (lane == 0 && OUT != kWalkPhi) {  // a diagnostic's potential walk is not a step's walk
-    atomicAdd(&P->stat_visits, (unsigned long long)st_visits);
-    atomicAdd(&P->stat_pops, (unsigned long long)st_pops);
-    atomicAdd(&P->stat_m2p, (unsigned long long)st_m2p);
-    atomicAdd(&P->stat_p2p, (unsigned long long)st_p2p);
-    atomicAdd(&P->stat_m2l, (unsigned long long)st_m2l);
-    atomicAdd(&P->stat_p2p_slots, (unsigned long long)st_slots);
+  if (OUT != kWalkPhi && lane < 6) {
+    unsigned long long* const total[6] = {&P->stat_visits, &P->stat_pops, &P->stat_m2p,
+                                          &P->stat_p2p, &P->stat_m2l, &P->stat_p2p_slots};
+    if (S.stat[lane]) atomicAdd(total[lane], (unsigned long long)S.stat[lane]);
   }
 }
 
-template <int W, bool GRAV, bool QUAD, bool NBR, bool HILO, int OUT>
-static void walk(const Dev& d, const Cfg& c, cudaStream_t s) {
-  const int blocks = (d.ngroups + W - 1) / W;
-  const size_t smem = sizeof(WalkSmem<W>);
+// One class of groups: [first, first + count) of the group table, F warps to a group.
+template <int F, bool GRAV, bool QUAD, bool NBR, bool HILO, int OUT>
+static int walk_class(const Dev& d, const Cfg& c, int first, int count, cudaStream_t s) {
+  if (count <= 0) return 0;
+  const size_t smem = sizeof(WalkSmem<F>);
   static std::atomic<unsigned long long> attr{0};
-  smem_limit_per_device(k_tree_walk<W, GRAV, QUAD, NBR, HILO, OUT>, (int)smem, attr);
+  smem_limit_per_device(k_tree_walk<F, GRAV, QUAD, NBR, HILO, OUT>, (int)smem, attr);
   const State& st = d.s();
-  k_tree_walk<W, GRAV, QUAD, NBR, HILO, OUT><<<blocks, W * 32, smem, s>>>(
+  constexpr int most = WalkSmem<F>::STACK;
+  k_tree_walk<F, GRAV, QUAD, NBR, HILO, OUT><<<count, F * 32, smem, s>>>(
       d.body, st.pos_h, st.x, st.y, st.z, d.K, d.L, d.leaf_start, d.leaf_codes, d.segs, d.left, d.right, d.ncom,
       d.nbmin, d.nbmax, d.nq0, d.nq1, d.P, d.grav, d.nbr, d.nbr_cnt, d.nbr_cap, c.h_solve ? -1.0f : c.nbr_skin,
-      d.h0, d.groups, d.ngroups, c.walk_stack > 0 && c.walk_stack < TW_STACK ? c.walk_stack : TW_STACK,
+      d.h0, d.groups + first, c.walk_stack > 0 && c.walk_stack < most ? c.walk_stack : most,
       GRAV ? c.local_theta : 0.0f, GRAV ? half_leaf(d, c) : 0, d.hcom, d.hq0, d.hq1, d.hrc);
-}
-
-// Gravity (group MAC) fused with the neighbour lists; the traversal tile (warps per block) is a tuning choice.
-template <bool QUAD, int OUT>
-static void walk_fused(const Dev& d, const Cfg& c, cudaStream_t s) {
-  if (c.hilo) {
-    walk<4, true, QUAD, true, true, OUT>(d, c, s);
-    return;
-  }
-  switch (c.walk_warps) {
-    case 4: walk<4, true, QUAD, true, false, OUT>(d, c, s); break;
-    case 8: walk<8, true, QUAD, true, false, OUT>(d, c, s); break;
-    default: walk<2, true, QUAD, true, false, OUT>(d, c, s); break;
-  }
-}
-
-int launch_walk(const Dev& d, const Cfg& c, bool potential, cudaStream_t s) {
-  if (potential) {
-    if (c.quad) walk_fused<true, kWalkAccPhi>(d, c, s);
-    else walk_fused<false, kWalkAccPhi>(d, c, s);
-  } else {
-    if (c.quad) walk_fused<true, kWalkAcc>(d, c, s);
-    else walk_fused<false, kWalkAcc>(d, c, s);
-  }
   return 1;
+}
+
+template <bool GRAV, bool QUAD, bool NBR, bool HILO, int OUT>
+static int walk(const Dev& d, const Cfg& c, cudaStream_t s) {
+  const int wide = d.ngroups - d.shared_groups;
+  return walk_class<1, GRAV, QUAD, NBR, HILO, OUT>(d, c, d.shared_groups, wide, s) +
+         walk_class<4, GRAV, QUAD, NBR, HILO, OUT>(d, c, 0, d.shared_groups, s);
+}
+
+template <bool QUAD, int OUT>
+static int walk_fused(const Dev& d, const Cfg& c, cudaStream_t s) {
+  return c.hilo ? walk<true, QUAD, true, true, OUT>(d, c, s) : walk<true, QUAD, true, false, OUT>(d, c, s);
+}
+
+// Gravity (group MAC) fused with the neighbour lists.
+int launch_walk(const Dev& d, const Cfg& c, bool potential, cudaStream_t s) {
+  if (potential) return c.quad ? walk_fused<true, kWalkAccPhi>(d, c, s) : walk_fused<false, kWalkAccPhi>(d, c, s);
+  return c.quad ? walk_fused<true, kWalkAcc>(d, c, s) : walk_fused<false, kWalkAcc>(d, c, s);
 }
 
 // The potential alone, into .w of the gravity record, on the tree of the last evaluation (the energy
 // diagnostic after steps whose walks left it out). The group MAC and quadrupoles of the step's walk; without
 // the neighbour lists a node is near only when it overlaps the part's box.
 int launch_potential(const Dev& d, const Cfg& c, cudaStream_t s) {
-  if (c.hilo) {
-    if (c.quad) walk<4, true, true, false, true, kWalkPhi>(d, c, s);
-    else walk<4, true, false, false, true, kWalkPhi>(d, c, s);
-  } else {
-    if (c.quad) walk<4, true, true, false, false, kWalkPhi>(d, c, s);
-    else walk<4, true, false, false, false, kWalkPhi>(d, c, s);
-  }
-  return 1;
+  if (c.hilo) return c.quad ? walk<true, true, false, true, kWalkPhi>(d, c, s) : walk<true, false, false, true, kWalkPhi>(d, c, s);
+  return c.quad ? walk<true, true, false, false, kWalkPhi>(d, c, s) : walk<true, false, false, false, kWalkPhi>(d, c, s);
 }
 
 // Neighbour lists only (when gravity is not the tree).
 int launch_neighbours(const Dev& d, const Cfg& c, cudaStream_t s) {
-  walk<4, false, false, true, false, kWalkAcc>(d, c, s);
-  return 1;
+  return walk<false, false, true, false, kWalkAcc>(d, c, s);
 }
 
 }  // namespace sphb

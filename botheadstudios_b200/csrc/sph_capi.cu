@@ -336,27 +336,34 @@ sph_status upload_impl(sph_ctx* ctx, const SphParticle48* particles, const uint3
   d.segbits = nimp > 1 ? bits_for(nimp) : 0;
   // segment table: each impact's leaves are K-particle buckets from its first particle
   std::vector<Seg> table((size_t)d.nseg + 1);
-  uint32_t L = 0, groups = 0;
+  uint32_t L = 0, groups = 0, shared = 0;
   const uint32_t per = (uint32_t)group_leaves(d.K);
+  const auto leaves = [&](uint32_t k) { return (off[k + 1] - off[k] + (uint32_t)d.K - 1) / (uint32_t)d.K; };
+  const auto is_shared = [&](uint32_t k) { return off[k + 1] - off[k] <= kSharedWalkMax; };
+  for (uint32_t k = 0; k < nimp; ++k)
+    if (is_shared(k)) shared += (leaves(k) + per - 1) / per;
+  d.shared_groups = (int)shared;  // their groups come first in the group table
+  d.ngroups = 0;
   for (uint32_t k = 0; k <= nimp; ++k) {
     Seg& g = table[k];
     std::memset(&g, 0, sizeof(g));
     g.off = k < nimp ? off[k] : nu;
     g.loff = L;
-    g.pad = groups;
     g.sig_bits = 0x7f800000u;
     for (int a = 0; a < 3; ++a) g.bbox[a] = 0xffffffffu;
     g.soft2 = k < nimp ? soft[k] * soft[k] : 0.0f;
     g.skin = ctx->hp.skin_wide;  // new positions: the first rebuild's solve gets the wide skin
     g.dt = ctx->hp.dt_fixed;
     if (k < nimp) {
-      const uint32_t leaves = (off[k + 1] - off[k] + (uint32_t)d.K - 1) / (uint32_t)d.K;
-      L += leaves;
-      groups += (leaves + per - 1) / per;
+      const uint32_t n_groups = (leaves(k) + per - 1) / per;
+      uint32_t& next = is_shared(k) ? groups : shared;
+      g.pad = next;
+      next += n_groups;
+      d.ngroups += (int)n_groups;
+      L += leaves(k);
     }
   }
   d.L = (int)L;
-  d.ngroups = (int)groups;
   ctx->n_eos = ne;
   if (!keep_eos) {
     Eos etab[kMaxMaterials];
@@ -518,7 +525,6 @@ sph_status sph_create(const sph_config* cfg, uint32_t capacity, sph_ctx** out) {
   ctx->kc.skin = ctx->kc.h_solve ? (cfg->h_skin > 0.0f ? cfg->h_skin : 0.05f) : 0.0f;
   ctx->kc.mac = (int)cfg->mac;
   ctx->kc.blk = cfg->block_threads ? (int)cfg->block_threads : 256;
-  ctx->kc.walk_warps = cfg->walk_warps ? (int)cfg->walk_warps : 2;
   if (cfg->device >= 0) {
     cudaError_t de = cudaSetDevice(cfg->device);
     if (de != cudaSuccess) {
@@ -1471,6 +1477,7 @@ sph_status sph_dem_replace(sph_dem* dem, const SphGrain80* grains, uint32_t n) {
   d.cur = 0;
   d.L = n ? (int)((n + d.K - 1) / d.K) : 0;
   d.ngroups = (d.L + group_leaves(d.K) - 1) / group_leaves(d.K);
+  d.shared_groups = n <= kSharedWalkMax ? d.ngroups : 0;
   d.nseg = 1;
   d.segbits = 0;
   dem->stepped = false;

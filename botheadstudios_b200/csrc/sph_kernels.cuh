@@ -165,6 +165,7 @@ struct Dev {
   float2* hrc = nullptr;        // [L] opening radii of the two halves (size/θ + |centre − COM|)
   uint2* groups = nullptr;      // [L] walk groups: (first leaf, last leaf) of runs of 32/K leaves of one impact
   int ngroups = 0;              // number of groups
+  int shared_groups = 0;        // ... of which the first are walked by several warps each (kSharedWalkMax)
   unsigned* nbr = nullptr;      // interleaved neighbour lists [n/32][nbr_cap][32]
   unsigned* nbr_cnt = nullptr;  // [n]
   unsigned nbr_cap = 0;
@@ -203,7 +204,6 @@ struct Cfg {
   int mac = 0;          // 0 group walk, 1 per-particle reference walk
   float nbr_skin = 0.0f;  // list inflation without the h-solve (grain contacts: a superset, cut exactly later)
   int blk = 256;        // threads per block of the per-particle gather kernels (density, h-solve, forces)
-  int walk_warps = 2;   // warps per block of the fused walk (2, 4 or 8)
   int learned = 0;      // smoothing lengths proposed by the MLP, checked, iterated only where rejected
   int divv = 0;         // the force pass also writes ∇·v (the learned proposal or its recording needs it)
   int walk_stack = 0;   // traversal-stack limit of the walks (0: their full stacks); for testing the overflow path
@@ -226,6 +226,7 @@ int launch_dem_contacts(const Dev& d, const DemParams& p, float4* acc, cudaStrea
 int launch_dem_integrate(const Dev& d, const DemParams& p, const float4* acc, cudaStream_t s);
 
 // ---- segments and tree -----------------------------------------------------------------------------
+constexpr uint32_t kSharedWalkMax = 32768;                // impacts up to this size: several warps walk for a group
 constexpr int group_leaves(int K) { return 32 / K; }      // leaves of a walk group
 int launch_segments(const Dev& d, cudaStream_t s);        // leaf starts and walk groups from the segment table
 int launch_segments_single(const Dev& d, float soft2, double dt, cudaStream_t s);  // one segment, on the device

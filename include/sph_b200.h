@@ -85,13 +85,14 @@ typedef struct sph_config {
                              and replays it (phase timing is not recorded for replayed substeps) */
   uint32_t block_threads; /* threads per block of the density, h-solve and force kernels: 64..1024, a multiple of
                              32; 0 = 256 */
-  uint32_t walk_warps;    /* warps per block of the fused gravity + neighbour walk: 2, 4 or 8; 0 = 2 */
+  uint32_t walk_warps;    /* 2, 4 or 8; 0 = 2. Accepted for callers that set it: the walk picks the warps it gives a
+                             group of particles by the impact's size */
   float h_skin;           /* SOLVE/LEARNED: neighbour lists are built at h·(1 + h_skin) and h moves at most that far
                              per rebuild, once the previous solve converged (residual <= 10·h_tol); after an
                              upload or an unconverged solve the skin is 0.15. 0 = 0.05 (at most 0.5) */
-  uint32_t walk_stack;    /* traversal-stack entries a walk may use (per warp in GROUP mode, 1,280 there; per
-                             particle in PARTICLE mode, 64 there as in bh_gravity.wgsl:336); 0 = all of them. A
-                             smaller limit is for testing the overflow path: children that do not fit are
+  uint32_t walk_stack;    /* traversal-stack entries a walk may use (per group in GROUP mode, 768 there, 2,560 in
+                             impacts of at most 32,768 particles; per particle in PARTICLE mode, 64 there as in
+                             bh_gravity.wgsl:336); 0 = all of them. A smaller limit is for testing the overflow path: children that do not fit are
                              skipped and SPH_ERR_OVERFLOW is raised through sph_diag (the reference drops them
                              silently, bh_gravity.wgsl:388-391) */
   float local_theta;      /* GROUP mode: an accepted node whose COM lies beyond r_g/local_theta of the group's
@@ -406,7 +407,7 @@ uint32_t sph_dem_count(const sph_dem* dem);
  * first call before any stream capture (a first call inside a capture returns SPH_ERR_STATE). Every call
  * uses the same array, so calls whose work overlaps on the GPU (different streams, or different host threads
  * on one device) race and corrupt each other's results: order them on one stream. If the traversal stack
- * (1,280 nodes per warp) overflows, every output is NaN. A CUDA error already pending on the calling thread
+ * (4,096 nodes for 32 points) overflows, every output is NaN. A CUDA error already pending on the calling thread
  * is left in place and returns SPH_ERR_CUDA before any work is enqueued. */
 sph_status sph_gravity_tree_noalloc(const void* d_bodies4, uint32_t n, double G, float softening, float theta,
                                     uint32_t leaf_size, uint32_t multipole, void* d_acc4, void* stream);
