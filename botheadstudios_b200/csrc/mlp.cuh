@@ -15,9 +15,9 @@ constexpr int MLP_W1 = 0, MLP_B1 = MLP_W1 + MLP_IN * MLP_H, MLP_W2 = MLP_B1 + ML
               MLP_XS = MLP_XM + MLP_IN, MLP_YM = MLP_XS + MLP_IN, MLP_YS = MLP_YM + 1, MLP_TOTAL = MLP_YS + 1;
 static_assert(MLP_TRAIN == 4801 && MLP_TOTAL == 4819, "parameter block");
 
-// Weights as the kernels read them: BF16 matrices row by row (the kernels copy them into the tcgen05 operand layout; K padded to
-// 16 for the first layer), FP32 biases and normalisation, W3 rounded to BF16 and held as FP32.
-struct MlpPacked {
+// Weights as the kernels read them: BF16 matrices in the tcgen05 operand layout (K-major without swizzle: 8-row × 16-byte
+// core matrices; K padded to 16 for the first layer), FP32 biases and normalisation, W3 rounded to BF16 and held as FP32.
+struct alignas(16) MlpPacked {
   __nv_bfloat16 w1t[MLP_H * 16];     // [out][in], in 8..15 zero
   __nv_bfloat16 w2t[MLP_H * MLP_H];  // [out][in]
   __nv_bfloat16 w2[MLP_H * MLP_H];   // [in][out]
@@ -28,7 +28,7 @@ struct MlpPacked {
   float ym, ys;
 };
 
-// FP32 parameter block → packed weights (one block of 256 threads).
+// FP32 parameter block → packed weights.
 int launch_mlp_pack(const float* params, MlpPacked* out, cudaStream_t s);
 
 // Inputs of the proposal, per particle, from the state of the step that is being taken (before the drift's
@@ -49,14 +49,20 @@ int launch_mlp_propose(const Dev& d, const MlpPacked* w, const MlpFeatureArgs& f
 // wait gave up (the outputs are then NaN).
 int launch_mlp_forward(const MlpPacked* w, const float* x, int n, float* out, unsigned* err, cudaStream_t s);
 
-// One training minibatch on tcgen05: forward + backward over rows idx[0..m) of (x, t), gradients of the mean
-// squared error on the normalised target (divided by `denom`) accumulated into grad[4801], the summed squared
-// error into *loss; *err |= 1 if a tensor-core barrier wait gave up (the tile's gradients are then incomplete).
+// One training minibatch on tcgen05: forward + backward over rows idx[0..m) of (x, t). Each of its CTAs writes its share
+// of the gradient of the mean squared error on the normalised target (divided by `denom`) and of the summed squared
+// error, 4,802 values, to part (mlp_part_floats(m) floats); *err |= 1 if a tensor-core barrier wait gave up (a share is
+// then missing).
+size_t mlp_part_floats(int m);
 int launch_mlp_train_batch(const MlpPacked* w, const float* x, const float* t, const unsigned* idx, int m,
-                           float denom, float* grad, float* loss, unsigned* err, cudaStream_t s);
+                           float denom, float* part, unsigned* err, cudaStream_t s);
 
-// Adam on the trainable parameters (FP32 master copy), step count `step` (1-based).
-int launch_mlp_adam(float* params, const float* grad, float* m, float* v, int step, float lr, float b1, float b2,
-                    float eps, float wd, cudaStream_t s);
+// The shares of a minibatch of m rows, summed: gradient[4801], then the summed squared error.
+int launch_mlp_reduce(const float* part, int m, float* grad_loss, cudaStream_t s);
+
+// Adam on the trainable parameters (FP32 master copy) with a minibatch's shares, step count `step` (1-based); adds its
+// summed squared error to *loss and packs the new weights.
+int launch_mlp_adam(float* params, const float* part, int batch, float* m, float* v, MlpPacked* w, float* loss, int step,
+                    float lr, float b1, float b2, float eps, float wd, cudaStream_t s);
 
 }  // namespace sphb
