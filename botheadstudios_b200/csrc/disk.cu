@@ -14,13 +14,12 @@
 //      2.44 R (ρ_remnant / ρ_clump)^(1/3); the Moon candidate is the heaviest bound clump outside it.
 //
 // Here every step is a kernel over the impact's particle range of the state (already contiguous per impact):
-// deterministic two-pass f64 reductions; the radius sort is the tree's 8-bit LSD radix sort over the exact
-// f64 bit patterns of the radii; the 85 % crossing is a block prefix over tile masses, then over the crossing
-// tile's particles; classification writes per-block partials and an order-preserving compaction of the disk;
-// the friends-of-friends search sorts the disk by a lexicographic cell key (cell edge just above the linking
+// deterministic two-pass f64 reductions; the 85 % crossing is a selection over the exact f64 bit patterns of the
+// radii, its running masses summed as integers; classification writes per-block partials and an order-preserving
+// compaction of the disk; the friends-of-friends search sorts the disk by a lexicographic cell key (cell edge just above the linking
 // length, so every linked pair lies in the 3 × 3 column of z-runs around a particle), and one warp per
-// particle scans its partners and unites linked pairs with a lock-free union-find (hooking the larger root
-// under the smaller with atomicCAS, path halving; parent[i] <= i always, so every walk ends); clumps are
+// particle scans its partners and unites linked pairs with a lock-free union-find (a root is hooked under a
+// node of lower rank with atomicCAS, path halving; ranks fall along every path, so every walk ends); clumps are
 // contiguous after a radix sort by root; one block per clump sums its moments; the self-potential is split
 // into 128 × 128 tile pairs of the clump's pair triangle, each summed in f64 by one block, then reduced per
 // clump in a fixed order. The per-particle arithmetic that decides a classification (radii, periapsis, pair
@@ -34,6 +33,8 @@
 
 namespace sphb {
 
+struct RadiusSelect;
+
 struct DiskWork {
   int cap = 0;
   void* base = nullptr;
@@ -41,7 +42,7 @@ struct DiskWork {
   unsigned* vals[2] = {nullptr, nullptr};
   void* sort_work = nullptr;
   double* part = nullptr;   // [kDmBlocks][kDmVals] block partials
-  double* tsum = nullptr;   // [tiles] mass of each radius-sorted tile
+  RadiusSelect* sel = nullptr;  // the mass-fraction crossing's counters
   double* scal = nullptr;   // [S_COUNT]
   unsigned* cnt = nullptr;  // [C_COUNT]
   unsigned* bcnt = nullptr; // [kDmBlocks] disk particles per block, then their output offsets
@@ -77,15 +78,17 @@ constexpr int kDmThreads = 256;
 constexpr int kDmBlocks = 592;  // 4 × 148 SMs; block b reduces the b-th contiguous chunk of the impact
 constexpr int kDmVals = 8;
 constexpr int kPeRows = 128;    // particles per self-potential row
-constexpr int kTile = 2048;     // radius-sorted tile of the crossing walk
-constexpr unsigned kCellBias = 1u << 20, kCellMax = (1u << 21) - 1u;
+constexpr int kSelBits = 12, kSelBins = 1 << kSelBits;  // digits of the crossing's selection
+constexpr int kSelBrute = 1024;  // candidates that one block ranks directly
+constexpr int kCellBits = 21;  // of a cell coordinate, at most
 constexpr int kUnionTries = 1 << 16;
 constexpr unsigned long long kMaxUnits = 1ull << 28;  // self-potential tile pairs (2 GB of partial sums)
 constexpr double kPiD = 3.14159265358979323846;
 constexpr unsigned kMaxPlacements = 256;
 
 enum { S_M = 0, S_COM = 1, S_VCOM = 4, S_RREM = 7, S_MREM = 8, S_LINK = 9, S_RHOREM = 10, S_CAT = 11, S_COUNT = 24 };
-enum { C_NDISK = 0, C_NCLUMP = 1, C_SEL = 2, C_ERR = 3, C_UNITS64 = 4, C_MINH = 6, C_COUNT = 8 };  // u64 in 4-5
+enum { C_NDISK = 0, C_NCLUMP = 1, C_SEL = 2, C_ERR = 3, C_UNITS64 = 4, C_MINH = 6, C_CELLBITS = 7, C_COUNT = 8 };
+// (u64 in 4-5; the disk's extent before its cell bits in 7)
 // body-bulk slots: the current centre and radius, the latest selection's centre and mass, its crossing radius
 // and running mass, the mass of every particle of the body
 enum { BB_C = 0, BB_R = 3, BB_CN = 4, BB_MN = 7, BB_RN = 8, BB_M = 10 };
@@ -127,11 +130,28 @@ __device__ __forceinline__ float3 pos_f32(const State& st, unsigned t) {
   return make_float3((float)st.x[t], (float)st.y[t], (float)st.z[t]);
 }
 
+}  // namespace
+
+// The selection's counters: zero before each use.
+struct RadiusSelect {
+  unsigned long long hist[2][kSelBins];  // weight in each bin of the first and of the second digit
+  unsigned long long base[2];            // the weight before the crossing bin of each
+  unsigned bin[2];                       // those bins
+  unsigned done[3];                      // blocks that finished each pass
+  unsigned count;                        // candidates listed
+  unsigned amax;                         // the largest |coordinate| of the points (float bits)
+  unsigned pad;
+};
+
+namespace {
+
 // ---- 1. mass, centre of mass, bulk velocity ----------------------------------------------------------
 __global__ void __launch_bounds__(kDmThreads) k_dm_moments(State st, unsigned off, unsigned m, unsigned chunk,
-                                                           double* __restrict__ part, float4* __restrict__ pm) {
+                                                           double* __restrict__ part, float4* __restrict__ pm,
+                                                           RadiusSelect* __restrict__ sel) {
   __shared__ double s[kDmThreads / 32][kDmVals];
   double a[kDmVals] = {0, 0, 0, 0, 0, 0, 0, 0};
+  float amax = 0.0f;
   const unsigned b0 = blockIdx.x * chunk, b1 = min(m, b0 + chunk);
   for (unsigned i = b0 + threadIdx.x; i < b1; i += kDmThreads) {
     const unsigned t = off + i;
@@ -139,6 +159,7 @@ __global__ void __launch_bounds__(kDmThreads) k_dm_moments(State st, unsigned of
     const float4 v = st.vel_u[t];
     const double mm = st.mass[t];
     pm[i] = make_float4(p.x, p.y, p.z, st.mass[t]);  // positions and masses for the remnant radius
+    amax = fmaxf(amax, fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z))));
     a[0] += mm;
     a[1] += (double)p.x * mm;  // f32 × f32 products are exact in f64
     a[2] += (double)p.y * mm;
@@ -148,6 +169,8 @@ __global__ void __launch_bounds__(kDmThreads) k_dm_moments(State st, unsigned of
     a[6] += (double)v.z * mm;
     a[7] += (double)st.pos_h[t].w;
   }
+  amax = warp_max(amax);
+  if ((threadIdx.x & 31) == 0) atomicMax(&sel->amax, __float_as_uint(amax));
   block_sum(a, s);
   if (threadIdx.x == 0)
     for (int k = 0; k < kDmVals; ++k) part[blockIdx.x * kDmVals + k] = a[k];
@@ -170,125 +193,207 @@ __global__ void k_dm_moments_final(const double* __restrict__ part, int nb, doub
   }
 }
 
-// ---- 2. radii about a centre, their sort, the mass-fraction crossing ------------------------------------
-// Shared by the remnant radius (85 % of an impact's mass) and the bulk radius of a body (98 %). pm holds the
+// ---- 2. radii about a centre, the mass-fraction crossing --------------------------------------------------
+// Shared by the remnant radius (85 % of an impact's mass) and the bulk radius of a body (98 %): the point whose running
+// mass, in radius order about the centre (equal radii in index order), first reaches frac of the total. pm holds the
 // points' f32 positions and masses; the radius is the exact f64 distance from the centre.
-__global__ void k_dm_radius(const float4* __restrict__ pm, unsigned m, const double* __restrict__ centre,
-                            unsigned long long* __restrict__ keys, unsigned* __restrict__ vals) {
-  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  const float4 p = pm[i];
+//
+// A selection, not a sort: a first pass sums the weights in 4,096 bins of the radius's leading bits (64 bins an octave,
+// down from a bound on the radii), a second one in the 4,096 bins of its next 12 bits inside the bin where the running
+// weight crosses, a third lists the points of the crossing bin there, some ten of a million, and one block ranks those.
+// Weights are integers, so the sums do not depend on their order and equal masses sum exactly. Bound by three readings of the points; a radix sort of the 64-bit radii, the masses
+// gathered in its order and two prefixes took 226 µs at 1,024,845 points, the three passes take 52.
+__device__ __forceinline__ unsigned long long radius_bits(float4 p, const double* __restrict__ centre) {
   const double dx = __dsub_rn((double)p.x, centre[0]), dy = __dsub_rn((double)p.y, centre[1]),
                dz = __dsub_rn((double)p.z, centre[2]);
-  const double r = __dsqrt_rn(dsq3(dx, dy, dz));
-  keys[i] = (unsigned long long)__double_as_longlong(r);  // r >= 0: the bit pattern orders like the value
-  vals[i] = i;
+  return (unsigned long long)__double_as_longlong(__dsqrt_rn(dsq3(dx, dy, dz)));  // r >= 0: ordered like the value
+}
+// A point's weight: its mass in units of a power of two that puts the total between 2^61 and 2^62, so masses above
+// 2^-38 of the total are whole. Without mass (or with one that is no number) every point weighs one: the first crosses.
+__device__ __forceinline__ double sel_scale(double total) {
+  return total > 0.0 && total < 1e300 ? __longlong_as_double((2107ll - (__double_as_longlong(total) >> 52)) << 52) : 0.0;
+}
+__device__ __forceinline__ unsigned long long sel_weight(float m, double scale) {
+  return scale > 0.0 ? __double2ull_rn((double)m * scale) : 1ull;
+}
+__device__ __forceinline__ unsigned long long sel_target(double frac, double total, double scale) {
+  const unsigned long long t = scale > 0.0 ? __double2ull_ru(__dmul_rn(frac, total) * scale) : 1ull;
+  return t > 0ull ? t : 1ull;
+}
+// First digit: the leading bits below those of `bound`, larger radii first; the last bin takes everything below.
+__device__ __forceinline__ unsigned sel_bin(unsigned long long key, unsigned long long bound) {
+  const unsigned long long hi = bound >> 46, k = key >> 46;
+  const unsigned long long d = hi > k ? hi - k : 0ull;
+  return d < (unsigned long long)(kSelBins - 1) ? (unsigned)d : (unsigned)(kSelBins - 1);
 }
 
-__global__ void __launch_bounds__(kDmThreads) k_dm_tile_mass(const float4* __restrict__ pm, unsigned m,
-                                                             const unsigned* __restrict__ order,
-                                                             double* __restrict__ tsum) {
-  __shared__ double s[kDmThreads / 32][kDmVals];
-  double a[kDmVals] = {0, 0, 0, 0, 0, 0, 0, 0};
-  const unsigned b0 = blockIdx.x * kTile, b1 = min(m, b0 + kTile);
-  for (unsigned i = b0 + threadIdx.x; i < b1; i += kDmThreads) a[0] += (double)pm[order[i]].w;
-  block_sum(a, s);
-  if (threadIdx.x == 0) tsum[blockIdx.x] = a[0];
-}
-
-// Block-wide exclusive scan of one double per thread (fixed association). Returns the block total in `total`.
-__device__ __forceinline__ double block_exclusive_scan_d(double v, double* s_warp, double& total) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  double incl = v;
+// The bin of h (shared memory; in order of radius: from the last one down when `down`) where a running weight that starts
+// at `base` reaches the target, or the sum if that falls short; base becomes the weight before that bin. The whole block.
+__device__ unsigned sel_cross(const unsigned long long* h, bool down, unsigned long long& base, unsigned long long target) {
+  __shared__ unsigned long long s_sum[kDmThreads / 32], s_base;
+  __shared__ unsigned s_bin;
+  constexpr int PER = kSelBins / kDmThreads;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  unsigned long long sum = 0ull;
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {  // (each lane starts elsewhere in its run: no bank conflicts)
+    const int i = t * PER + ((k + t) & (PER - 1));
+    sum += h[down ? kSelBins - 1 - i : i];
+  }
+  unsigned long long incl = sum;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const double t = __shfl_up_sync(SPH_FULL_MASK, incl, o);
-    if (lane >= o) incl += t;
+    const unsigned long long v = __shfl_up_sync(SPH_FULL_MASK, incl, o);
+    if (lane >= o) incl += v;
   }
-  if (lane == 31) s_warp[w] = incl;
+  if (lane == 31) s_sum[w] = incl;
   __syncthreads();
-  if (w == 0) {
-    const double x = lane < nw ? s_warp[lane] : 0.0;
-    double xi = x;
+  unsigned long long before = base + incl - sum, total = base;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const double t = __shfl_up_sync(SPH_FULL_MASK, xi, o);
-      if (lane >= o) xi += t;
+  for (int k = 0; k < kDmThreads / 32; ++k) {
+    if (k < w) before += s_sum[k];
+    total += s_sum[k];
+  }
+  target = target < total ? target : total;
+  if (before < target && before + sum >= target) {  // one thread
+    int i = t * PER;
+    for (;; ++i) {  // ends within the run: its sum reaches the target
+      const unsigned long long v = h[down ? kSelBins - 1 - i : i];
+      if (before + v >= target || i == t * PER + PER - 1) break;
+      before += v;
     }
-    if (lane < nw) s_warp[lane] = xi - x;
-    if (lane == 31) s_warp[32] = xi;
+    s_bin = (unsigned)(down ? kSelBins - 1 - i : i);
+    s_base = before;
   }
   __syncthreads();
-  const double res = s_warp[w] + incl - v;
-  total = s_warp[32];
+  base = s_base;
+  const unsigned bin = s_bin;
   __syncthreads();
-  return res;
+  return bin;
 }
 
-// The mass-fraction crossing in radius order: a prefix over the tile masses finds the crossing tile, a prefix
-// over its points (two per thread) the first one whose running mass reaches frac·(*total). out[0] = its
-// radius, out[1] = the running mass there (the last radius and the total when rounding keeps the sum short).
-// One block of 1024 threads.
-__global__ void __launch_bounds__(1024) k_dm_cross(const float4* __restrict__ pm, unsigned m, int tiles,
-                                                   const unsigned long long* __restrict__ keys,
-                                                   const unsigned* __restrict__ order, const double* __restrict__ tsum,
-                                                   const double* __restrict__ total_mass, double frac,
-                                                   double* __restrict__ out) {
-  __shared__ double s_warp[33];
-  __shared__ unsigned s_tile, s_idx;
-  __shared__ double s_base, s_cum;
-  const double M = *total_mass, thr = frac * M;
-  const unsigned per = ((unsigned)tiles + blockDim.x - 1) / blockDim.x, t0 = threadIdx.x * per;
-  double local = 0.0;
-  for (unsigned k = 0; k < per; ++k)
-    if (t0 + k < (unsigned)tiles) local += tsum[t0 + k];
-  if (threadIdx.x == 0) {
-    s_tile = 0xffffffffu;
-    s_idx = 0xffffffffu;
-  }
-  double total;
-  double cum = block_exclusive_scan_d(local, s_warp, total);  // synchronises, so s_tile is initialised
-  unsigned mine = 0xffffffffu;
-  for (unsigned k = 0; k < per && t0 + k < (unsigned)tiles; ++k) {
-    if (cum + tsum[t0 + k] >= thr) {
-      mine = t0 + k;
-      atomicMin(&s_tile, mine);
-      break;
+// The crossing point among the n listed ones, by one block: its radius to out[0], the running mass there to out[1]. Up to
+// kSelBrute candidates are ranked directly, by (radius, index); more (a great many equal radii) by further digits of both.
+__device__ void sel_rank(unsigned long long* h, const float4* __restrict__ pm, unsigned n, double scale,
+                         unsigned long long target, unsigned long long base, const unsigned long long* list_key,
+                         const unsigned* list_idx, double* __restrict__ out) {
+  const unsigned t = threadIdx.x;
+  if (n <= (unsigned)kSelBrute) {
+    unsigned long long *s_key = h, *s_w = h + kSelBrute;
+    unsigned* s_idx = reinterpret_cast<unsigned*>(h + 2 * kSelBrute);
+    for (unsigned i = t; i < n; i += kDmThreads) {
+      s_key[i] = __ldcg(list_key + i);
+      s_idx[i] = __ldcg(list_idx + i);
+      s_w[i] = sel_weight(pm[s_idx[i]].w, scale);
     }
-    cum += tsum[t0 + k];
-  }
-  __syncthreads();
-  // the crossing tile is the first crossing of its owner's run, so the owner's running mass is its base
-  if (mine != 0xffffffffu && mine == s_tile) s_base = cum;
-  if (threadIdx.x == 0 && s_tile == 0xffffffffu) s_base = total;
-  __syncthreads();
-  // walk the particles from the crossing tile on (normally within it; rounding may push it to the next)
-  double base = s_base;
-  for (unsigned start = (s_tile == 0xffffffffu ? (unsigned)tiles : s_tile) * kTile; start < m; start += kTile) {
-    const unsigned i0 = start + 2u * threadIdx.x;
-    const double v0 = i0 < m ? (double)pm[order[i0]].w : 0.0;
-    const double v1 = i0 + 1u < m ? (double)pm[order[i0 + 1u]].w : 0.0;
-    double tile_total;
-    const double ex = block_exclusive_scan_d(v0 + v1, s_warp, tile_total);
-    const double c0 = base + ex + v0, c1 = c0 + v1;
-    if (i0 < m && c0 >= thr) atomicMin(&s_idx, i0);
-    else if (i0 + 1u < m && c1 >= thr) atomicMin(&s_idx, i0 + 1u);
     __syncthreads();
-    if (s_idx != 0xffffffffu) {
-      if (threadIdx.x == (s_idx - start) >> 1) s_cum = s_idx == i0 ? c0 : c1;
-      break;
+    for (unsigned i = t; i < n; i += kDmThreads) {
+      const unsigned long long key = s_key[i], w = s_w[i];
+      unsigned long long before = base, total = base;
+      for (unsigned k = 0; k < n; ++k) {
+        if (s_key[k] < key || (s_key[k] == key && s_idx[k] < s_idx[i])) before += s_w[k];
+        total += s_w[k];
+      }
+      const unsigned long long goal = target < total ? target : total;
+      if (before < goal && before + w >= goal) {  // one candidate
+        out[0] = __longlong_as_double((long long)key);
+        out[1] = scale > 0.0 ? (double)(before + w) / scale : 0.0;
+      }
     }
-    base += tile_total;
+    return;
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double r_rem = __longlong_as_double((long long)keys[m - 1]), m_rem = M;
-    if (s_idx != 0xffffffffu) {
-      r_rem = __longlong_as_double((long long)keys[s_idx]);
-      m_rem = s_cum;
+  // composite digits, most significant first: the 64 bits of the radius, then the 32 of the index
+  unsigned long long pk = 0ull;
+  unsigned pi = 0u;
+  for (int d = 0; d < 9; ++d) {
+    const bool on_key = d < 6;
+    const int shift = on_key ? 52 - kSelBits * d : 20 - kSelBits * (d - 6);  // 52, 40, .. -8; 20, 8, -4
+    const int lo = shift > 0 ? shift : 0, width = shift >= 0 ? kSelBits : kSelBits + shift, top = lo + width;
+    for (int k = t; k < kSelBins; k += kDmThreads) h[k] = 0ull;
+    __syncthreads();
+    for (unsigned i = t; i < n; i += kDmThreads) {
+      const unsigned long long k = __ldcg(list_key + i);
+      const unsigned x = __ldcg(list_idx + i);
+      const bool in = on_key ? top >= 64 || (k >> top) == (pk >> top) : k == pk && (top >= 32 || (x >> top) == (pi >> top));
+      if (in) atomicAdd(&h[(on_key ? (unsigned)(k >> lo) : x >> lo) & ((1u << width) - 1u)], sel_weight(pm[x].w, scale));
     }
-    out[0] = r_rem;
-    out[1] = m_rem;
+    __syncthreads();
+    const unsigned bin = sel_cross(h, false, base, target);
+    if (on_key) pk |= (unsigned long long)bin << lo;
+    else pi |= bin << lo;
+  }
+  if (t == 0) {
+    out[0] = __longlong_as_double((long long)pk);
+    out[1] = scale > 0.0 ? (double)(base + sel_weight(pm[pi].w, scale)) / scale : 0.0;
+  }
+}
+
+// Pass 0: weights by the first digit; the radii are kept for the other passes. Pass 1: by the second digit inside the
+// crossing bin. Pass 2: the points of the crossing bin of both digits into the list. The last block of a pass to finish
+// finds the pass's crossing bin (at the start of the next pass, in every block, that took 10 µs a pass), or ranks the list.
+template <int PASS>
+__global__ void __launch_bounds__(kDmThreads) k_dm_select_radius(const float4* __restrict__ pm, unsigned m, unsigned chunk,
+                                                                 const double* __restrict__ centre,
+                                                                 const double* __restrict__ total_mass, double frac,
+                                                                 unsigned long long* __restrict__ keys,
+                                                                 RadiusSelect* sel, unsigned long long* list_key,
+                                                                 unsigned* list_idx, double* __restrict__ out) {
+  __shared__ unsigned long long h[kSelBins];
+  __shared__ int s_last;
+  const double M = *total_mass, scale = sel_scale(M);
+  // the centre is a mean of the points, so no radius is above 2 sqrt(3) times their largest coordinate
+  const unsigned long long bound = (unsigned long long)__double_as_longlong(4.0 * (double)__uint_as_float(sel->amax));
+  const unsigned long long target = sel_target(frac, M, scale);
+  const unsigned a = PASS > 0 ? sel->bin[0] : 0u, b = PASS > 1 ? sel->bin[1] : 0u;
+  const bool whole = a == (unsigned)(kSelBins - 1);  // the bin of everything far below the bound has no second digit
+  if (PASS == 0) {
+    for (int k = threadIdx.x; k < kSelBins; k += kDmThreads) h[k] = 0ull;
+    __syncthreads();
+  }
+  const unsigned b0 = blockIdx.x * chunk, b1 = min(m, b0 + chunk);
+#pragma unroll 4
+  for (unsigned i = b0 + threadIdx.x; i < b1; i += kDmThreads) {
+    if (PASS == 0) {
+      const float4 p = pm[i];
+      const unsigned long long key = radius_bits(p, centre);
+      keys[i] = key;
+      atomicAdd(&h[sel_bin(key, bound)], sel_weight(p.w, scale));
+    } else {
+      const unsigned long long key = keys[i];
+      if (sel_bin(key, bound) == a) {
+        const unsigned e = whole ? 0u : (unsigned)(key >> 34) & (kSelBins - 1);
+        if (PASS == 1) {
+          atomicAdd(&sel->hist[1][e], sel_weight(pm[i].w, scale));  // (few points: no block's share of its own)
+        } else if (e == b) {
+          const unsigned at = atomicAdd(&sel->count, 1u);
+          list_key[at] = key;
+          list_idx[at] = i;
+        }
+      }
+    }
+  }
+  if (PASS == 0) {
+    __syncthreads();
+    for (int k = threadIdx.x; k < kSelBins; k += kDmThreads)
+      if (h[k]) atomicAdd(&sel->hist[0][k], h[k]);
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(&sel->done[PASS], 1u) == gridDim.x - 1u;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  if (PASS < 2) {
+    for (int k = threadIdx.x; k < kSelBins; k += kDmThreads) h[k] = __ldcg(&sel->hist[PASS][k]);
+    __syncthreads();
+    unsigned long long base = PASS == 0 ? 0ull : sel->base[0];
+    const unsigned bin = sel_cross(h, PASS == 0, base, target);
+    if (threadIdx.x == 0) {
+      sel->bin[PASS] = bin;
+      sel->base[PASS] = base;
+    }
+  } else {
+    sel_rank(h, pm, __ldcg(&sel->count), scale, target, sel->base[1], list_key, list_idx, out);
   }
 }
 
@@ -319,39 +424,53 @@ __device__ __forceinline__ int classify(int variant, double px, double py, doubl
 __global__ void __launch_bounds__(kDmThreads) k_dm_classify(State st, unsigned off, unsigned m, unsigned chunk,
                                                             int variant, double G, const double* __restrict__ scal,
                                                             unsigned char* __restrict__ cat,
-                                                            double* __restrict__ part, unsigned* __restrict__ bcnt) {
+                                                            double* __restrict__ part, unsigned* __restrict__ bcnt,
+                                                            unsigned* __restrict__ cnt) {
   __shared__ double s[kDmThreads / 32][kDmVals];
   double a[kDmVals] = {0, 0, 0, 0, 0, 0, 0, 0};
   const double cx = scal[S_COM], cy = scal[S_COM + 1], cz = scal[S_COM + 2];
   const double ux = scal[S_VCOM], uy = scal[S_VCOM + 1], uz = scal[S_VCOM + 2];
   const double mu = G * scal[S_MREM], r_rem = scal[S_RREM];
   const unsigned b0 = blockIdx.x * chunk, b1 = min(m, b0 + chunk);
-  unsigned ndisk = 0;
-  for (unsigned base = b0; base < b1; base += kDmThreads) {
-    const unsigned i = base + threadIdx.x;
-    int is_disk = 0;
-    if (i < b1) {
-      const unsigned t = off + i;
-      const float3 p = pos_f32(st, t);
-      const float4 v = st.vel_u[t];
-      const int c = classify(variant, __dsub_rn((double)p.x, cx), __dsub_rn((double)p.y, cy),
-                             __dsub_rn((double)p.z, cz), __dsub_rn((double)v.x, ux), __dsub_rn((double)v.y, uy),
-                             __dsub_rn((double)v.z, uz), mu, r_rem);
-      const int k = (c == 1 ? 0 : c == 2 ? 2 : 4) + (st.prov[t] == 0u ? 0 : 1);
-      cat[i] = (unsigned char)k;
-      const double mm = st.mass[t];
+  float extent = 0.0f;  // of the disk particles from the centre, along an axis
+#pragma unroll 2
+  for (unsigned i = b0 + threadIdx.x; i < b1; i += kDmThreads) {
+    const unsigned t = off + i;
+    const float3 p = pos_f32(st, t);
+    const float4 v = st.vel_u[t];
+    const double dx = __dsub_rn((double)p.x, cx), dy = __dsub_rn((double)p.y, cy), dz = __dsub_rn((double)p.z, cz);
+    const int c = classify(variant, dx, dy, dz, __dsub_rn((double)v.x, ux), __dsub_rn((double)v.y, uy),
+                           __dsub_rn((double)v.z, uz), mu, r_rem);
+    const int k = (c == 1 ? 0 : c == 2 ? 2 : 4) + (st.prov[t] == 0u ? 0 : 1);
+    cat[i] = (unsigned char)k;
+    const double mm = st.mass[t];
 #pragma unroll
-      for (int j = 0; j < 6; ++j) a[j] += j == k ? mm : 0.0;
-      if (c == 1) a[6] += (double)st.pos_h[t].w;
-      is_disk = c == 1;
+    for (int j = 0; j < 6; ++j) a[j] += j == k ? mm : 0.0;
+    if (c == 1) {
+      a[6] += (double)st.pos_h[t].w;
+      a[7] += 1.0;
+      extent = fmaxf(extent, __double2float_ru(fmax(fabs(dx), fmax(fabs(dy), fabs(dz)))));
     }
-    ndisk += (unsigned)__syncthreads_count(is_disk);
   }
+  extent = warp_max(extent);
+  if ((threadIdx.x & 31) == 0 && extent > 0.0f) atomicMax(&cnt[C_CELLBITS], __float_as_uint(extent));
   block_sum(a, s);
   if (threadIdx.x == 0) {
     for (int k = 0; k < kDmVals; ++k) part[blockIdx.x * kDmVals + k] = a[k];
-    bcnt[blockIdx.x] = ndisk;
+    bcnt[blockIdx.x] = (unsigned)a[7];
   }
+}
+
+// Cells an edge just above the linking length wide: a linked pair differs by at most one cell per axis even after
+// the f32 subtraction of the tool's distance.
+__device__ __forceinline__ double inv_cell(double link) { return 1.0 / (link * (1.0 + 0x1p-20)); }
+// Bits of a cell coordinate that hold every disk particle, from the largest distance along an axis from the centre: the
+// sort reads no more digits than the disk's extent needs (27-30 bits of key for a ring, three passes instead of seven).
+__device__ __forceinline__ int cell_bits(float extent, double link) {
+  const double cells = (double)extent * inv_cell(link) + 1.0;
+  int b = 1;
+  while (b < kCellBits && !(cells < (double)(1u << (b - 1)))) ++b;
+  return b;
 }
 
 __global__ void __launch_bounds__(1024) k_dm_classify_final(const double* __restrict__ part, int nb, unsigned m,
@@ -376,6 +495,7 @@ __global__ void __launch_bounds__(1024) k_dm_classify_final(const double* __rest
     for (int k = 0; k < 6; ++k) scal[S_CAT + k] = t[k];
     const double mean_h = variant == 0 ? (total ? t[6] / (double)total : 0.0) : scal[S_CAT + 7] / (double)m;
     scal[S_LINK] = link_factor * mean_h;
+    cnt[C_CELLBITS] = (unsigned)cell_bits(__uint_as_float(cnt[C_CELLBITS]), link_factor * mean_h);
     const double disk = t[0] + t[1];
     out[0] = disk > 0.0 ? 100.0 * t[0] / disk : 0.0;
     out[1] = disk;
@@ -388,18 +508,19 @@ __global__ void __launch_bounds__(1024) k_dm_classify_final(const double* __rest
 }
 
 // ---- 4. friends-of-friends over the disk ----------------------------------------------------------------
-__device__ __forceinline__ unsigned cell_coord(double x, double c, double inv_cs) {
-  const double q = floor((x - c) * inv_cs) + (double)kCellBias;
+__device__ __forceinline__ unsigned cell_coord(double x, double c, double inv_cs, int bits) {
+  const double q = floor((x - c) * inv_cs) + (double)(1u << (bits - 1));
+  const unsigned top = (1u << bits) - 1u;
   if (!(q > 0.0)) return 0u;  // clamping only merges far cells: linked pairs stay within one cell per axis
-  return q >= (double)kCellMax ? kCellMax : (unsigned)q;
+  return q >= (double)top ? top : (unsigned)q;
 }
-__device__ __forceinline__ unsigned long long cell_key(unsigned ix, unsigned iy, unsigned iz) {
-  return ((unsigned long long)ix << 42) | ((unsigned long long)iy << 21) | (unsigned long long)iz;
+__device__ __forceinline__ unsigned long long cell_key(unsigned ix, unsigned iy, unsigned iz, int bits) {
+  return ((unsigned long long)ix << (2 * bits)) | ((unsigned long long)iy << bits) | (unsigned long long)iz;
 }
-
-// Order-preserving compaction of the disk particles (block b writes from its offset in chunk order).
+// Order-preserving compaction of the disk particles (block b writes from its offset in chunk order, a thread its own run
+// of the chunk: one scan a block).
 __global__ void __launch_bounds__(kDmThreads) k_dm_compact(State st, const float* __restrict__ rho, unsigned off,
-                                                           unsigned m, unsigned chunk,
+                                                           unsigned m, unsigned chunk, int bits,
                                                            const unsigned char* __restrict__ cat,
                                                            const unsigned* __restrict__ boff,
                                                            const double* __restrict__ scal, float4* __restrict__ dpos,
@@ -408,27 +529,25 @@ __global__ void __launch_bounds__(kDmThreads) k_dm_compact(State st, const float
                                                            unsigned* __restrict__ vals) {
   __shared__ unsigned s_warp[33];
   const double cx = scal[S_COM], cy = scal[S_COM + 1], cz = scal[S_COM + 2];
-  // cell edge just above the linking length: a linked pair differs by at most one cell per axis even after
-  // the f32 subtraction of the tool's distance
-  const double inv_cs = 1.0 / (scal[S_LINK] * (1.0 + 0x1p-20));
+  const double inv_cs = inv_cell(scal[S_LINK]);
   const unsigned b0 = blockIdx.x * chunk, b1 = min(m, b0 + chunk);
-  unsigned run = boff[blockIdx.x];
-  for (unsigned base = b0; base < b1; base += kDmThreads) {
-    const unsigned i = base + threadIdx.x;
-    const unsigned f = (i < b1 && cat[i] < 2) ? 1u : 0u;
-    unsigned total;
-    const unsigned o = run + block_exclusive_scan(f, s_warp, total);
-    if (f) {
-      const unsigned t = off + i;
-      const float3 p = pos_f32(st, t);
-      const float4 v = st.vel_u[t];
-      dpos[o] = make_float4(p.x, p.y, p.z, st.pos_h[t].w);
-      dvel[o] = make_float4(v.x, v.y, v.z, st.mass[t]);
-      drp[o] = make_float2(rho[t], __uint_as_float(st.prov[t]));
-      keys[o] = cell_key(cell_coord(p.x, cx, inv_cs), cell_coord(p.y, cy, inv_cs), cell_coord(p.z, cz, inv_cs));
-      vals[o] = o;
-    }
-    run += total;
+  const unsigned per = chunk / kDmThreads, i0 = b0 + threadIdx.x * per, i1 = min(b1, i0 + per);
+  unsigned mine = 0u, total;
+  for (unsigned i = i0; i < i1; ++i) mine += cat[i] < 2 ? 1u : 0u;
+  unsigned o = boff[blockIdx.x] + block_exclusive_scan(mine, s_warp, total);
+  if (!mine) return;
+  for (unsigned i = i0; i < i1; ++i) {
+    if (cat[i] >= 2) continue;
+    const unsigned t = off + i;
+    const float3 p = pos_f32(st, t);
+    const float4 v = st.vel_u[t];
+    dpos[o] = make_float4(p.x, p.y, p.z, st.pos_h[t].w);
+    dvel[o] = make_float4(v.x, v.y, v.z, st.mass[t]);
+    drp[o] = make_float2(rho[t], __uint_as_float(st.prov[t]));
+    keys[o] = cell_key(cell_coord(p.x, cx, inv_cs, bits), cell_coord(p.y, cy, inv_cs, bits),
+                       cell_coord(p.z, cz, inv_cs, bits), bits);
+    vals[o] = o;
+    ++o;
   }
 }
 
@@ -448,7 +567,12 @@ __global__ void k_dm_gather(unsigned n, const unsigned* __restrict__ order, cons
   }
 }
 
-// Root of x with path halving. parent[v] <= v for every v and the walk strictly decreases, so it ends.
+// A node's rank, a fixed shuffle of the indices (multiplication by an odd number): roots are hooked by rank, since the
+// particles are sorted in space and hooking by index makes chains across a whole ring. And the node of a rank.
+__device__ __forceinline__ unsigned uf_rank(unsigned x) { return x * 2654435761u; }
+__device__ __forceinline__ unsigned uf_node(unsigned r) { return r * 244002641u; }
+
+// Root of x with path halving. A parent's rank is below its child's and the walk strictly falls, so it ends.
 __device__ __forceinline__ unsigned uf_find(unsigned* parent, unsigned x) {
   volatile unsigned* p = parent;
   unsigned nx = p[x];
@@ -461,13 +585,16 @@ __device__ __forceinline__ unsigned uf_find(unsigned* parent, unsigned x) {
   return x;
 }
 
+// Unites the groups of a and b, which were seen as roots. A root is hooked under a node of lower rank, wherever that
+// node's own root is by then: ranks fall along every path, so no cycle can form.
 __device__ __forceinline__ bool uf_unite(unsigned* parent, unsigned a, unsigned b) {
   for (int k = 0; k < kUnionTries; ++k) {
-    a = uf_find(parent, a);
-    b = uf_find(parent, b);
     if (a == b) return true;
-    const unsigned hi = a > b ? a : b, lo = a > b ? b : a;
+    const bool up = uf_rank(a) > uf_rank(b);
+    const unsigned hi = up ? a : b, lo = up ? b : a;
     if (atomicCAS(&parent[hi], hi, lo) == hi) return true;  // a failed hook means hi gained a parent
+    a = uf_find(parent, hi);
+    b = uf_find(parent, lo);
   }
   return false;
 }
@@ -489,42 +616,65 @@ __device__ __forceinline__ unsigned lower_bound_u64(const unsigned long long* k,
   return lo;
 }
 
-// One warp per particle a: lanes 0-8 find the nine (x, y) columns' z-runs in the sorted cell keys, then the
-// warp scans each run's partners after a, 32 at a time; a linked partner whose root differs from a's is united.
-__global__ void __launch_bounds__(kDmThreads) k_dm_link(unsigned n, int variant,
+// One warp per particle a: lanes 0-8 find the starts of the nine (x, y) columns' z-runs in the sorted cell keys, lanes
+// 9-17 their ends; then the warp scans the runs' partners after a as one sequence, 32 at a time; a linked partner whose
+// root differs from a's is united. Bound by the latency of the unions of one ring-wide group, whose roots change under
+// many warps at once: searches and scan alone take 19 µs for 22,840 particles, with the unions hooked by index, each
+// lane's partner under a's root by turns, 145 µs, by rank under the batch's lowest root 64-79.
+__global__ void __launch_bounds__(kDmThreads) k_dm_link(unsigned n, int variant, int bits,
                                                         const unsigned long long* __restrict__ skeys,
                                                         const float4* __restrict__ dpos,
                                                         const double* __restrict__ scal,
                                                         unsigned* __restrict__ parent, unsigned* __restrict__ cnt) {
   const unsigned lane = threadIdx.x & 31u;
   const unsigned nwarps = (gridDim.x * blockDim.x) >> 5;
+  const unsigned top = (1u << bits) - 1u;
   const double link = scal[S_LINK], link2 = link * link;
   bool ok = true;
   for (unsigned a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; a + 1u < n; a += nwarps) {
     const unsigned long long ka = skeys[a], knext = skeys[a + 1u];
-    const unsigned ix = (unsigned)(ka >> 42), iy = (unsigned)(ka >> 21) & kCellMax, iz = (unsigned)ka & kCellMax;
-    unsigned j0 = 0, j1 = 0;
-    if (lane < 9u) {
-      const int cx = (int)ix + (int)(lane / 3u) - 1, cy = (int)iy + (int)(lane % 3u) - 1;
-      if (cx >= 0 && cx <= (int)kCellMax && cy >= 0 && cy <= (int)kCellMax) {
-        const unsigned long long lo = cell_key((unsigned)cx, (unsigned)cy, iz ? iz - 1u : 0u);
-        const unsigned long long hi = cell_key((unsigned)cx, (unsigned)cy, iz < kCellMax ? iz + 1u : kCellMax);
-        if (hi >= knext) {  // partners come after a in the order, so each pair is tested once
-          j0 = max(lower_bound_u64(skeys, n, lo), a + 1u);
-          j1 = lower_bound_u64(skeys, n, hi + 1ull);
-        }
+    const float4 pa = dpos[a];
+    const unsigned ix = (unsigned)(ka >> (2 * bits)), iy = (unsigned)(ka >> bits) & top, iz = (unsigned)ka & top;
+    const bool high = lane >= 9u;
+    const unsigned col = high ? lane - 9u : lane;
+    unsigned at = 0u;  // first partner of the column, or the one past its last
+    if (lane < 18u) {
+      const int cx = (int)ix + (int)(col / 3u) - 1, cy = (int)iy + (int)(col % 3u) - 1;
+      if (cx >= 0 && cx <= (int)top && cy >= 0 && cy <= (int)top) {
+        const unsigned long long lo = cell_key((unsigned)cx, (unsigned)cy, iz ? iz - 1u : 0u, bits);
+        const unsigned long long hi = cell_key((unsigned)cx, (unsigned)cy, iz < top ? iz + 1u : top, bits);
+        if (hi >= knext)  // partners come after a in the order, so each pair is tested once
+          at = max(lower_bound_u64(skeys, n, high ? hi + 1ull : lo), a + 1u);
       }
     }
-    const float4 pa = dpos[a];
-    const unsigned ra = uf_find(parent, a);
-    for (int c = 0; c < 9; ++c) {
-      const unsigned b0 = __shfl_sync(SPH_FULL_MASK, j0, c), b1 = __shfl_sync(SPH_FULL_MASK, j1, c);
-      for (unsigned j = b0 + lane; j < b1; j += 32u)
-        if (pair_d2(variant, pa, dpos[j]) <= link2) {
-          const unsigned rb = uf_find(parent, j);
-          // equal roots: already one group (a root never stops being one while its group is unmerged)
-          if (rb != ra) ok &= uf_unite(parent, ra, rb);
-        }
+    const unsigned end = __shfl_down_sync(SPH_FULL_MASK, at, 9);
+    const unsigned len = lane < 9u ? end - at : 0u;
+    unsigned upto = len;  // partners in this column and those before it
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) {
+      const unsigned t = __shfl_up_sync(SPH_FULL_MASK, upto, o);
+      if (lane >= (unsigned)o) upto += t;
+    }
+    const unsigned total = __shfl_sync(SPH_FULL_MASK, upto, 8);
+    const unsigned shift = at - (upto - len);  // partner k of the sequence is particle k + its column's shift
+    unsigned ra = total ? uf_find(parent, a) : a;
+    for (unsigned k0 = 0; k0 < total; k0 += 32u) {
+      const unsigned k = k0 + lane;
+      unsigned j = 0u;
+#pragma unroll
+      for (int c = 0; c < 9; ++c) {
+        const unsigned before = __shfl_sync(SPH_FULL_MASK, upto - len, c), sh = __shfl_sync(SPH_FULL_MASK, shift, c);
+        const unsigned count = __shfl_sync(SPH_FULL_MASK, len, c);
+        if (k - before < count) j = k + sh;
+      }
+      const bool linked = k < total && pair_d2(variant, pa, dpos[j]) <= link2;
+      if (!__any_sync(SPH_FULL_MASK, linked)) continue;
+      // all that is linked goes under the batch's root of lowest rank: the lanes hook different roots, one of them a's
+      const unsigned rb = linked ? uf_find(parent, j) : ra;
+      const unsigned low = uf_node(__reduce_min_sync(SPH_FULL_MASK, min(uf_rank(rb), uf_rank(ra))));
+      if (linked && rb != ra && rb != low) ok &= uf_unite(parent, rb, low);
+      if (lane == 0u && ra != low) ok &= uf_unite(parent, ra, low);
+      ra = low;
     }
   }
   if (!ok) atomicOr(&cnt[C_ERR], 1u);
@@ -534,7 +684,7 @@ __global__ void k_dm_roots(unsigned n, unsigned* __restrict__ parent, unsigned* 
                            unsigned long long* __restrict__ keys, unsigned* __restrict__ vals) {
   const unsigned a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= n) return;
-  const unsigned r = uf_find(parent, a);  // the smallest index of a's group
+  const unsigned r = uf_find(parent, a);
   atomicAdd(&gcnt[r], 1u);
   keys[a] = r;
   vals[a] = a;
@@ -542,8 +692,8 @@ __global__ void k_dm_roots(unsigned n, unsigned* __restrict__ parent, unsigned* 
 
 // ---- 5. clumps ------------------------------------------------------------------------------------------
 __global__ void k_dm_clumps(unsigned n, const unsigned long long* __restrict__ skeys,
-                            const unsigned* __restrict__ gcnt, uint4* __restrict__ clump,
-                            unsigned* __restrict__ cnt) {
+                            const unsigned* __restrict__ order, const unsigned* __restrict__ gcnt,
+                            uint4* __restrict__ clump, unsigned* __restrict__ cnt) {
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const unsigned r = (unsigned)skeys[i];
@@ -551,7 +701,7 @@ __global__ void k_dm_clumps(unsigned n, const unsigned long long* __restrict__ s
   const unsigned s = gcnt[r];
   if (s < 2u) return;
   const unsigned c = atomicAdd(&cnt[C_NCLUMP], 1u);
-  clump[c] = make_uint4(i, s, r, 0u);
+  clump[c] = make_uint4(i, s, order[i], 0u);  // (the sort is stable: the group's smallest index)
 }
 
 // One block per clump: mass, centre of mass, volume, target mass, then the internal kinetic energy.
@@ -566,7 +716,8 @@ __global__ void __launch_bounds__(kDmThreads) k_dm_clump_stats(const unsigned* _
   const unsigned ncl = cnt[C_NCLUMP];
   for (unsigned c = blockIdx.x; c < ncl; c += gridDim.x) {
     const uint4 cl = clump[c];
-    double a[kDmVals] = {0, 0, 0, 0, 0, 0, 0, 0}, b[kDmVals] = {0, 0, 0, 0, 0, 0, 0, 0};
+    double a[kDmVals] = {0, 0, 0, 0, 0, 0, 0, 0}, target = 0.0;
+#pragma unroll 4
     for (unsigned j = threadIdx.x; j < cl.y; j += kDmThreads) {
       const unsigned t = cl.x + j;
       const float4 p = dpos[t], v = dvel[t];
@@ -581,10 +732,9 @@ __global__ void __launch_bounds__(kDmThreads) k_dm_clump_stats(const unsigned* _
       a[6] += (double)p.z * mm;
       const double rho = variant == 0 ? (double)rp.x : (double)fmaxf(rp.x, 1.0f);  // gpu_sph.rs:450
       a[7] += mm / rho;
-      b[0] += __float_as_uint(rp.y) == 0u ? mm : 0.0;
+      target += __float_as_uint(rp.y) == 0u ? mm : 0.0;
     }
     block_sum(a, s);
-    block_sum(b, s);
     if (threadIdx.x == 0) {
       for (int k = 0; k < 3; ++k) s_cv[k] = a[1 + k] / a[0];
       double* o = cstat + (size_t)c * 8;
@@ -593,17 +743,20 @@ __global__ void __launch_bounds__(kDmThreads) k_dm_clump_stats(const unsigned* _
       o[2] = a[5] / a[0];
       o[3] = a[6] / a[0];
       o[4] = a[7];
-      o[5] = b[0];
     }
     __syncthreads();
-    double k3[kDmVals] = {0, 0, 0, 0, 0, 0, 0, 0};
+    double k3[kDmVals] = {0, target, 0, 0, 0, 0, 0, 0};
     const double cvx = s_cv[0], cvy = s_cv[1], cvz = s_cv[2];
+#pragma unroll 4
     for (unsigned j = threadIdx.x; j < cl.y; j += kDmThreads) {
       const float4 v = dvel[cl.x + j];
       k3[0] += 0.5 * (double)v.w * dsq3((double)v.x - cvx, (double)v.y - cvy, (double)v.z - cvz);
     }
     block_sum(k3, s);
-    if (threadIdx.x == 0) cstat[(size_t)c * 8 + 6] = k3[0];
+    if (threadIdx.x == 0) {
+      cstat[(size_t)c * 8 + 5] = k3[1];
+      cstat[(size_t)c * 8 + 6] = k3[0];
+    }
   }
 }
 
@@ -736,8 +889,8 @@ __global__ void __launch_bounds__(kDmThreads) k_dm_select(const unsigned* __rest
                                                           const double* __restrict__ cstat,
                                                           const double* __restrict__ scal, int variant, double G,
                                                           double roche, double rho_fallback, double* __restrict__ out) {
-  __shared__ double s_m[kDmThreads], s_e[kDmThreads];
-  __shared__ unsigned s_root[kDmThreads], s_n[kDmThreads], s_bound[kDmThreads], s_cl[kDmThreads];
+  __shared__ double s_m[kDmThreads / 32], s_e[kDmThreads / 32];
+  __shared__ unsigned s_root[kDmThreads / 32], s_n[kDmThreads / 32], s_bound[kDmThreads / 32], s_cl[kDmThreads / 32];
   const unsigned ncl = cnt[C_NCLUMP];
   const double cx = scal[S_COM], cy = scal[S_COM + 1], cz = scal[S_COM + 2];
   const double r_rem = scal[S_RREM], rho_rem = scal[S_RHOREM];
@@ -763,23 +916,37 @@ __global__ void __launch_bounds__(kDmThreads) k_dm_select(const unsigned* __rest
       bn = cl.y;
     }
   }
-  s_m[threadIdx.x] = bm;
-  s_e[threadIdx.x] = be;
-  s_root[threadIdx.x] = broot;
-  s_n[threadIdx.x] = bn;
-  s_bound[threadIdx.x] = nb;
-  s_cl[threadIdx.x] = nc;
+  // the best of each warp, then of the warps (the larger mass, the smaller root: any order gives the same)
+  const auto better = [&](double m, double e, unsigned root, unsigned n) {
+    if (m > bm || (m == bm && m > 0.0 && root < broot)) {
+      bm = m;
+      be = e;
+      broot = root;
+      bn = n;
+    }
+  };
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    better(__shfl_xor_sync(SPH_FULL_MASK, bm, o), __shfl_xor_sync(SPH_FULL_MASK, be, o),
+           __shfl_xor_sync(SPH_FULL_MASK, broot, o), __shfl_xor_sync(SPH_FULL_MASK, bn, o));
+    nb += __shfl_xor_sync(SPH_FULL_MASK, nb, o);
+    nc += __shfl_xor_sync(SPH_FULL_MASK, nc, o);
+  }
+  const int w = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0) {
+    s_m[w] = bm;
+    s_e[w] = be;
+    s_root[w] = broot;
+    s_n[w] = bn;
+    s_bound[w] = nb;
+    s_cl[w] = nc;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int k = 1; k < kDmThreads; ++k) {
+    for (int k = 1; k < kDmThreads / 32; ++k) {
       nb += s_bound[k];
       nc += s_cl[k];
-      if (s_m[k] > bm || (s_m[k] == bm && s_m[k] > 0.0 && s_root[k] < broot)) {
-        bm = s_m[k];
-        be = s_e[k];
-        broot = s_root[k];
-        bn = s_n[k];
-      }
+      better(s_m[k], s_e[k], s_root[k], s_n[k]);
     }
     out[10] = bm;
     out[11] = bm > 0.0 ? 100.0 * be / bm : 0.0;
@@ -810,11 +977,13 @@ __device__ __forceinline__ bool bb_take(const State& st, unsigned t, unsigned pr
 
 __global__ void __launch_bounds__(kDmThreads) k_bb_count(State st, unsigned n, unsigned chunk, unsigned prov,
                                                          int clip, const double* __restrict__ bb,
-                                                         double* __restrict__ part, unsigned* __restrict__ bcnt) {
+                                                         double* __restrict__ part, unsigned* __restrict__ bcnt,
+                                                         RadiusSelect* __restrict__ sel) {
   __shared__ double s[kDmThreads / 32][kDmVals];
   double a[kDmVals] = {0, 0, 0, 0, 0, 0, 0, 0};
   const unsigned b0 = blockIdx.x * chunk, b1 = min(n, b0 + chunk);
   unsigned cnt = 0;
+  float amax = 0.0f;
   for (unsigned base = b0; base < b1; base += kDmThreads) {
     const unsigned t = base + threadIdx.x;
     const bool take = t < b1 && bb_take(st, t, prov, clip, bb);
@@ -825,9 +994,12 @@ __global__ void __launch_bounds__(kDmThreads) k_bb_count(State st, unsigned n, u
       a[1] += (double)p.x * mm;
       a[2] += (double)p.y * mm;
       a[3] += (double)p.z * mm;
+      amax = fmaxf(amax, fmaxf(fabsf(p.x), fmaxf(fabsf(p.y), fabsf(p.z))));
     }
     cnt += (unsigned)__syncthreads_count(take);
   }
+  amax = warp_max(amax);
+  if ((threadIdx.x & 31) == 0) atomicMax(&sel->amax, __float_as_uint(amax));
   block_sum(a, s);
   if (threadIdx.x == 0) {
     for (int k = 0; k < kDmVals; ++k) part[blockIdx.x * kDmVals + k] = a[k];
@@ -961,7 +1133,7 @@ bool work_reserve(DiskWork* w, int m, cudaStream_t s) {
   if (w->base) cudaFree(w->base);
   w->base = nullptr;
   w->cap = 0;
-  const size_t n = (size_t)(m < 1 ? 1 : m), half = n / 2 + 2, tiles = (n + kTile - 1) / kTile;
+  const size_t n = (size_t)(m < 1 ? 1 : m), half = n / 2 + 2;
   size_t sz = 0;
   auto take = [&](size_t bytes) {
     const size_t o = sz;
@@ -970,7 +1142,7 @@ bool work_reserve(DiskWork* w, int m, cudaStream_t s) {
   };
   const size_t o_k0 = take(8 * n), o_k1 = take(8 * n), o_v0 = take(4 * n), o_v1 = take(4 * n);
   const size_t o_sort = take(sort_work_bytes((int)n)), o_part = take(8 * kDmBlocks * kDmVals);
-  const size_t o_tsum = take(8 * tiles), o_scal = take(8 * S_COUNT), o_cnt = take(4 * C_COUNT);
+  const size_t o_sel = take(sizeof(RadiusSelect)), o_scal = take(8 * S_COUNT), o_cnt = take(4 * C_COUNT);
   const size_t o_bcnt = take(4 * kDmBlocks), o_cat = take(n);
   const size_t o_pm = take(16 * n), o_p0 = take(16 * n), o_p1 = take(16 * n), o_u0 = take(16 * n), o_u1 = take(16 * n);
   const size_t o_r0 = take(8 * n), o_r1 = take(8 * n), o_par = take(4 * n), o_g = take(4 * n);
@@ -991,7 +1163,7 @@ bool work_reserve(DiskWork* w, int m, cudaStream_t s) {
   w->vals[1] = (unsigned*)(b + o_v1);
   w->sort_work = b + o_sort;
   w->part = (double*)(b + o_part);
-  w->tsum = (double*)(b + o_tsum);
+  w->sel = (RadiusSelect*)(b + o_sel);
   w->scal = (double*)(b + o_scal);
   w->cnt = (unsigned*)(b + o_cnt);
   w->bcnt = (unsigned*)(b + o_bcnt);
@@ -1015,16 +1187,16 @@ bool work_reserve(DiskWork* w, int m, cudaStream_t s) {
 }
 
 // Radius of the point whose running mass, in radius order about `centre`, first reaches frac·(*total)
-// (out[0]) and that running mass (out[1]); every pointer is device memory; n >= 1.
+// (out[0]) and that running mass (out[1]); every pointer is device memory; n >= 1. sel: its counters zero, its amax set.
 int launch_radius_crossing(DiskWork* w, const float4* pm, unsigned n, const double* centre, const double* total,
                            double frac, double* out, cudaStream_t s) {
-  k_dm_radius<<<(n + 255) / 256, 256, 0, s>>>(pm, n, centre, w->keys[0], w->vals[0]);
-  int src = 0;
-  int L = 1 + launch_radix_sort(w->keys, w->vals, (int)n, 64, w->sort_work, w->cnt + C_ERR, src, s);
-  const int tiles = (int)((n + kTile - 1) / kTile);
-  k_dm_tile_mass<<<tiles, kDmThreads, 0, s>>>(pm, n, w->vals[src], w->tsum);
-  k_dm_cross<<<1, 1024, 0, s>>>(pm, n, tiles, w->keys[src], w->vals[src], w->tsum, total, frac, out);
-  return L + 2;
+  const unsigned chunk = ((n + kDmBlocks - 1) / kDmBlocks + kDmThreads - 1) / kDmThreads * kDmThreads;
+  const unsigned nb = (n + chunk - 1) / chunk;
+  unsigned long long *keys = w->keys[0], *list = w->keys[1];
+  k_dm_select_radius<0><<<nb, kDmThreads, 0, s>>>(pm, n, chunk, centre, total, frac, keys, w->sel, list, w->vals[0], out);
+  k_dm_select_radius<1><<<nb, kDmThreads, 0, s>>>(pm, n, chunk, centre, total, frac, keys, w->sel, list, w->vals[0], out);
+  k_dm_select_radius<2><<<nb, kDmThreads, 0, s>>>(pm, n, chunk, centre, total, frac, keys, w->sel, list, w->vals[0], out);
+  return 3;
 }
 
 }  // namespace
@@ -1051,38 +1223,41 @@ int disk_measure(const Dev& d, unsigned off, unsigned m, const DiskCfg& c, DiskW
   const unsigned chunk = ((m + kDmBlocks - 1) / kDmBlocks + kDmThreads - 1) / kDmThreads * kDmThreads;
   const int nb = (int)((m + chunk - 1) / chunk);
   cudaMemsetAsync(w->cnt, 0, 4 * C_COUNT, s);
-  k_dm_moments<<<nb, kDmThreads, 0, s>>>(st, off, m, chunk, w->part, w->pm);
+  cudaMemsetAsync(w->sel, 0, sizeof(RadiusSelect), s);
+  k_dm_moments<<<nb, kDmThreads, 0, s>>>(st, off, m, chunk, w->part, w->pm, w->sel);
   k_dm_moments_final<<<1, kDmThreads, 0, s>>>(w->part, nb, w->scal);
   L += 2;
   L += launch_radius_crossing(w, w->pm, m, w->scal + S_COM, w->scal + S_M, c.remnant_frac, w->scal + S_RREM, s);
-  k_dm_classify<<<nb, kDmThreads, 0, s>>>(st, off, m, chunk, c.variant, c.G, w->scal, w->cat, w->part, w->bcnt);
+  k_dm_classify<<<nb, kDmThreads, 0, s>>>(st, off, m, chunk, c.variant, c.G, w->scal, w->cat, w->part, w->bcnt, w->cnt);
   k_dm_classify_final<<<1, 1024, 0, s>>>(w->part, nb, m, c.variant, c.link_factor, w->bcnt, w->scal, w->cnt, w->out);
   L += 2;
-  unsigned nd = 0;
-  cudaMemcpyAsync(&nd, w->cnt + C_NDISK, 4, cudaMemcpyDeviceToHost, s);
+  unsigned flags[C_COUNT];
+  cudaMemcpyAsync(flags, w->cnt, sizeof(flags), cudaMemcpyDeviceToHost, s);
   cudaError_t e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {
     *err = cudaGetErrorString(e);
     return -2;
   }
+  const unsigned nd = flags[C_NDISK];
+  const int bits = (int)flags[C_CELLBITS];
   int src = 0;
   if (nd >= 2) {
-    k_dm_compact<<<nb, kDmThreads, 0, s>>>(st, d.rho, off, m, chunk, w->cat, w->bcnt, w->scal, w->dpos[0],
+    k_dm_compact<<<nb, kDmThreads, 0, s>>>(st, d.rho, off, m, chunk, bits, w->cat, w->bcnt, w->scal, w->dpos[0],
                                            w->dvel[0], w->drp[0], w->keys[0], w->vals[0]);
     L += 1;
-    L += launch_radix_sort(w->keys, w->vals, (int)nd, 63, w->sort_work, w->cnt + C_ERR, src, s);
+    L += launch_radix_sort(w->keys, w->vals, (int)nd, 3 * bits, w->sort_work, w->cnt + C_ERR, src, s);
     const unsigned gb = (nd + 255) / 256;
     k_dm_gather<<<gb, 256, 0, s>>>(nd, w->vals[src], w->dpos[0], w->dvel[0], w->drp[0], w->dpos[1], w->dvel[1],
                                    w->drp[1], w->parent, w->gcnt);
     const unsigned lb = (nd + 7) / 8;  // one warp per particle, grid-strided over at most 16 blocks per SM
-    k_dm_link<<<lb < 2368u ? lb : 2368u, kDmThreads, 0, s>>>(nd, c.variant, w->keys[src], w->dpos[1], w->scal,
+    k_dm_link<<<lb < 2368u ? lb : 2368u, kDmThreads, 0, s>>>(nd, c.variant, bits, w->keys[src], w->dpos[1], w->scal,
                                                              w->parent, w->cnt);
     k_dm_roots<<<gb, 256, 0, s>>>(nd, w->parent, w->gcnt, w->keys[0], w->vals[0]);
     L += 3;
     L += launch_radix_sort(w->keys, w->vals, (int)nd, bits_of(nd), w->sort_work, w->cnt + C_ERR, src, s);
     k_dm_gather<<<gb, 256, 0, s>>>(nd, w->vals[src], w->dpos[1], w->dvel[1], w->drp[1], w->dpos[0], w->dvel[0],
                                    w->drp[0], nullptr, nullptr);
-    k_dm_clumps<<<gb, 256, 0, s>>>(nd, w->keys[src], w->gcnt, w->clump, w->cnt);
+    k_dm_clumps<<<gb, 256, 0, s>>>(nd, w->keys[src], w->vals[src], w->gcnt, w->clump, w->cnt);
     const unsigned cb = nd / 2 < 1184u ? nd / 2 : 1184u;  // clumps <= nd / 2; blocks stride over them
     k_dm_clump_stats<<<cb, kDmThreads, 0, s>>>(w->cnt, w->clump, c.variant, w->dpos[0], w->dvel[0], w->drp[0],
                                                w->cstat);
@@ -1122,7 +1297,6 @@ int disk_measure(const Dev& d, unsigned off, unsigned m, const DiskCfg& c, DiskW
                                          c.rho_fallback, w->out);
     L += 1;
   }
-  unsigned flags[C_COUNT];
   cudaMemcpyAsync(out, w->out, 16 * sizeof(double), cudaMemcpyDeviceToHost, s);
   cudaMemcpyAsync(flags, w->cnt, sizeof(flags), cudaMemcpyDeviceToHost, s);
   e = cudaStreamSynchronize(s);
@@ -1175,7 +1349,8 @@ int body_bulk_impl(const Dev& d, unsigned prov, DiskWork* w, double* out5, unsig
   cudaMemsetAsync(w->bb, 0, 16 * sizeof(double), s);
   for (int round = 0; round < 3; ++round) {
     const int clip = round > 0;
-    k_bb_count<<<nb, kDmThreads, 0, s>>>(st, n, chunk, prov, clip, w->bb, w->part, w->bcnt);
+    cudaMemsetAsync(w->sel, 0, sizeof(RadiusSelect), s);
+    k_bb_count<<<nb, kDmThreads, 0, s>>>(st, n, chunk, prov, clip, w->bb, w->part, w->bcnt, w->sel);
     k_bb_scan<<<1, 1024, 0, s>>>(w->part, nb, round == 0, w->bcnt, w->bb, w->cnt);
     unsigned sel = 0;
     cudaMemcpyAsync(&sel, w->cnt + C_SEL, 4, cudaMemcpyDeviceToHost, s);
