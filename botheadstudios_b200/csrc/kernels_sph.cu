@@ -8,6 +8,9 @@
 // h_ij = ½(h_i + h_j). Here that set is enumerated once per tree build by a warp-cooperative walk of the
 // LBVH (node AABBs carry the subtree's max h) and stored as interleaved per-particle lists; r_ij is
 // computed with single-rounded operations so the set is bit-identical to the reference predicate.
+#include <type_traits>
+#include <utility>
+
 #include "sph_kernels.cuh"
 
 namespace sphb {
@@ -23,23 +26,33 @@ __device__ __forceinline__ float pair_r(float4 a, float4 b, float& rinv) {
 }
 __device__ __forceinline__ float pair_h(float hi, float hj) { return fmul(0.5f, fadd(hi, hj)); }
 
-// The gather kernels walk a particle's list kGather entries at a time: all of a chunk's indices are loaded,
-// then all of its neighbour records, before any is used, so each thread keeps kGather gathers in flight
-// instead of one dependent chain; the next chunk's indices are requested before this chunk's records, so the
-// list stream (HBM) overlaps the record gathers (mostly L1/L2) and the arithmetic. `lst` is the particle's
-// first list slot (entries 32 apart, interleaved); slots past the count read the sentinel record `sent` (a
-// massless particle outside every support), so a pair is evaluated without testing the count or the support
-// (kern_pair_bf vanishes outside it). The lists are read once per pass and streamed past the cache
-// (evict-first), so they do not push the neighbours' records out of L2.
+// The gather kernels sum a particle's list in kSums = 4 shares, entry k in share k mod 4, and add the shares in one
+// order: ((0 + 1) + (2 + 3)). Four neighbouring lanes hold the shares of a particle, or (density sums of larger batches)
+// two lanes two each: the same bits, so the choice may go by the size of the whole batch. Four lanes: the longest of 8
+// lists, not of 32, holds up a warp, a small impact has four times the warps, the last blocks of a launch are shorter,
+// and what one request gathers lies closer together (entries that follow one another in a list are mostly one leaf's, one
+// after the other in memory: the kernels' bound is the data path of the L1, then instruction issue). Two: half the
+// prologues, index streams and reductions. Against a lane to a particle a step with three contexts at once went from
+// 411 to 368 µs at 65,536 particles, from 773 to 694 at 131,072, 1,503 to 1,430 at 262,144; at 1M it is the same.
+//
+// A lane takes G of its entries at a time: all of a chunk's indices are loaded, then all of its neighbour records,
+// before any is used, so it keeps G gathers in flight instead of one dependent chain; the indices are requested two
+// chunks ahead of the records, so the list stream (HBM) overlaps the record gathers (mostly L1/L2) and the arithmetic.
+// `lst` is the particle's first list slot (entries 32 apart, interleaved); slots past the count read the sentinel record
+// `sent` (a massless particle outside every support), so a pair is evaluated without testing the count or the support
+// (kern_pair_bf vanishes outside it). The lists are read once per pass and streamed past the cache (evict-first), so
+// they do not push the neighbours' records out of L2.
+constexpr int kSums = 4;
 constexpr int kGather = 4;
-template <int G>
+template <int G, int L>
 __device__ __forceinline__ void list_chunk(const unsigned* __restrict__ lst, unsigned k0, unsigned c, unsigned sent,
                                            unsigned j[G]) {
 #pragma unroll
-  for (int u = 0; u < G; ++u) j[u] = k0 + u < c ? __ldcs(&lst[(size_t)(k0 + u) * 32u]) : sent;
+  for (int u = 0; u < G; ++u) j[u] = k0 + u * L < c ? __ldcs(&lst[(size_t)(k0 + u * L) * 32u]) : sent;
 }
 // Records of the chunk whose indices are in `jn` (k0 = its first slot); jn2 holds the next chunk's indices.
 // On return jn holds the next chunk's and jn2 the one after it: the list stays two chunks ahead of the records.
+template <int L>
 __device__ __forceinline__ void gather_pos_mass(const State& st, const unsigned* __restrict__ lst, unsigned k0,
                                                 unsigned c, unsigned sent, unsigned jn[kGather],
                                                 unsigned jn2[kGather], float4 pj[kGather], float mj[kGather]) {
@@ -49,12 +62,19 @@ __device__ __forceinline__ void gather_pos_mass(const State& st, const unsigned*
     j[u] = jn[u];
     jn[u] = jn2[u];
   }
-  list_chunk<kGather>(lst, k0 + 2 * kGather, c, sent, jn2);
+  list_chunk<kGather, L>(lst, k0 + 2 * kGather * L, c, sent, jn2);
 #pragma unroll
   for (int u = 0; u < kGather; ++u) {
     pj[u] = st.pos_h[j[u]];
     mj[u] = st.mass[j[u]];
   }
+}
+// The sum of a particle's shares, the same in each of its L lanes (v: this lane's shares, lowest first).
+template <int L>
+__device__ __forceinline__ float add_shares(const float v[kSums / L]) {
+  const float a = v[0] + __shfl_xor_sync(SPH_FULL_MASK, v[0], 1);
+  if constexpr (L == 2) return a + (v[1] + __shfl_xor_sync(SPH_FULL_MASK, v[1], 1));
+  else return a + __shfl_xor_sync(SPH_FULL_MASK, a, 2);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -71,47 +91,85 @@ __device__ __forceinline__ float4 eos_record(const Eos* __restrict__ eos, unsign
   return make_float4(m, rho, p / (rho * rho), c);
 }
 
-template <int KERNEL>
+// ρ_i and ∂ρ_i/∂h_i of a block's particles over their neighbour lists at their current h: the particle of a lane's list
+// is t, and thread k < blockDim / L gets the sums of particle tk (-1: none), so that what follows the sums (an EOS of some
+// hundred instructions) is done by one lane a particle in full warps. The whole block calls it; s: 2 blockDim / L floats.
+template <int KERNEL, int L>
+__device__ __forceinline__ void block_sums(int t, int tk, const State& st, const unsigned* __restrict__ nbr,
+                                           const unsigned* __restrict__ nbr_cnt, unsigned cap, unsigned sent, float* s,
+                                           float& rho, float& drho) {
+  static_assert(kGather % (kSums / L) == 0, "an entry's share is its place in the chunk");
+  const unsigned sub = threadIdx.x & (L - 1);
+  float r[kSums / L], d[kSums / L];  // Σ m_j W and Σ m_j ∂W/∂h_ij
+#pragma unroll
+  for (int k = 0; k < kSums / L; ++k) r[k] = d[k] = 0.0f;
+  if (t >= 0) {
+    const float4 pi = st.pos_h[t];
+    const unsigned c = min(nbr_cnt[t], cap);
+    const unsigned* lst = nbr + nbr_slot((unsigned)t, 0u, cap);
+    unsigned jn[kGather], jn2[kGather];
+    list_chunk<kGather, L>(lst, sub, c, sent, jn);
+    list_chunk<kGather, L>(lst, sub + kGather * L, c, sent, jn2);
+    for (unsigned k0 = sub; k0 < c; k0 += kGather * L) {
+      float4 pj[kGather];
+      float mj[kGather];
+      gather_pos_mass<L>(st, lst, k0, c, sent, jn, jn2, pj, mj);
+#pragma unroll
+      for (int u = 0; u < kGather; ++u) {
+        float ri, w, dwdr, dwdh;
+        const float q = pair_r(pi, pj[u], ri);
+        kern_pair_bf<KERNEL>(q, pair_h(pi.w, pj[u].w), w, dwdr, dwdh);
+        r[u & (kSums / L - 1)] += mj[u] * w;
+        d[u & (kSums / L - 1)] += mj[u] * dwdh;
+      }
+    }
+  }
+  float rs = add_shares<L>(r), ds = add_shares<L>(d);
+  const int np = blockDim.x / L;
+  if (sub == 0) {
+    s[threadIdx.x / L] = rs;
+    s[np + threadIdx.x / L] = ds;
+  }
+  __syncthreads();
+  if (tk < 0) return;
+  rs = s[threadIdx.x];
+  ds = s[np + threadIdx.x];
+  const float m = st.mass[tk];
+  float w, dwdr, dwdh;
+  kern_pair<KERNEL>(0.0f, st.pos_h[tk].w, w, dwdr, dwdh);
+  rho = m * w + rs;
+  drho = m * dwdh + 0.5f * ds;  // ∂h_ij/∂h_i = ½
+}
+constexpr int kMaxBlk = 1024;
+
+template <int KERNEL, int L>
 __global__ void k_density_eos(int n, State st, const unsigned* __restrict__ nbr,
                               const unsigned* __restrict__ nbr_cnt, unsigned cap, unsigned sent,
                               const Eos* __restrict__ eos, const DevParams* __restrict__ P,
                               float* __restrict__ rho, float4* __restrict__ fdata) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const float4 pi = st.pos_h[t];
-  const float m = st.mass[t];
-  float w, dwdr, dwdh;
-  kern_pair<KERNEL>(0.0f, pi.w, w, dwdr, dwdh);
-  float r_i = m * w;
-  const unsigned c = min(nbr_cnt[t], cap);
-  const unsigned* lst = nbr + nbr_slot((unsigned)t, 0u, cap);
-  unsigned jn[kGather], jn2[kGather];
-  list_chunk<kGather>(lst, 0u, c, sent, jn);
-  list_chunk<kGather>(lst, kGather, c, sent, jn2);
-  for (unsigned k0 = 0; k0 < c; k0 += kGather) {
-    float4 pj[kGather];
-    float mj[kGather];
-    gather_pos_mass(st, lst, k0, c, sent, jn, jn2, pj, mj);
-#pragma unroll
-    for (int u = 0; u < kGather; ++u) {
-      float ri;
-      const float r = pair_r(pi, pj[u], ri);
-      kern_pair_bf<KERNEL>(r, pair_h(pi.w, pj[u].w), w, dwdr, dwdh);
-      r_i += mj[u] * w;
-    }
-  }
+  __shared__ float s[2 * kMaxBlk / L];
+  const int np = blockDim.x / L, first = blockIdx.x * np;
+  const int g = first + (int)threadIdx.x / L, t = first + (int)threadIdx.x;
+  const bool mine = (int)threadIdx.x < np && t < n;
+  float r_i = 0.0f, d = 0.0f;
+  block_sums<KERNEL, L>(g < n ? g : -1, mine ? t : -1, st, nbr, nbr_cnt, cap, sent, s, r_i, d);
+  if (!mine) return;
   rho[t] = r_i;
-  fdata[t] = eos_record(eos, st.mat[t], m, r_i, st.vel_u[t].w, P);
+  fdata[t] = eos_record(eos, st.mat[t], st.mass[t], r_i, st.vel_u[t].w, P);
 }
 
+// Lanes a particle takes in the density sums. The density of 10,240 particles 10.7 µs with four lanes, 12.8 with two
+// (14.0 with one); a solve of two passes and the density 61 and 59 (62) at 32,768, 145 and 135 (142) at 180,000, 656 and
+// 562 (512) at 1,048,576 by itself, but with three contexts at once the step there is shorter with two than with one
+// (5,895 and 5,960).
+static int density_lanes(int n) { return n <= 20000 ? 4 : 2; }
+static int gather_blocks(int n, int blk, int lanes) { return (n + blk / lanes - 1) / (blk / lanes); }
+
 int launch_density_eos(const Dev& d, const Cfg& c, cudaStream_t s) {
-  const int blocks = (d.n + c.blk - 1) / c.blk;
-  if (c.kernel == 1)
-    k_density_eos<1><<<blocks, c.blk, 0, s>>>(d.n, d.s(), d.nbr, d.nbr_cnt, d.nbr_cap, d.sent, d.eos, d.P, d.rho,
-                                              d.fdata);
-  else
-    k_density_eos<0><<<blocks, c.blk, 0, s>>>(d.n, d.s(), d.nbr, d.nbr_cnt, d.nbr_cap, d.sent, d.eos, d.P, d.rho,
-                                              d.fdata);
+  const int lanes = density_lanes(d.n), blocks = gather_blocks(d.n, c.blk, lanes);
+  const auto kernel = c.kernel == 1 ? (lanes == 4 ? k_density_eos<1, 4> : k_density_eos<1, 2>)
+                                    : (lanes == 4 ? k_density_eos<0, 4> : k_density_eos<0, 2>);
+  kernel<<<blocks, c.blk, 0, s>>>(d.n, d.s(), d.nbr, d.nbr_cnt, d.nbr_cap, d.sent, d.eos, d.P, d.rho, d.fdata);
   return 1;
 }
 
@@ -132,8 +190,9 @@ int launch_eos_only(const Dev& d, cudaStream_t s) {
 // ∂rho_i/∂h_i = m_i ∂W(0,h_i)/∂h + Σ_j m_j ½ ∂W(r,h_ij)/∂h (Price 2012, J. Comput. Phys. 231, §3.2.1).
 // h may move inside the list's skin only; the residual |f|/rho is reduced to a device maximum.
 // ---------------------------------------------------------------------------------------------------
-// ρ_i and ∂ρ_i/∂h_i at the particle's current h over its neighbour list (the density sum of k_density_eos,
-// same terms in the same order).
+// ρ_i and ∂ρ_i/∂h_i at the particle's current h over its neighbour list, in one lane and in the list's order, for runs
+// with learned smoothing lengths: they compare the residual with a tolerance, where another order of the sum accepts other
+// particles, and the network takes ρ and h in 16 bits.
 template <int KERNEL>
 __device__ __forceinline__ void h_sums(int t, const State& st, const unsigned* __restrict__ nbr,
                                        const unsigned* __restrict__ nbr_cnt, unsigned cap, unsigned sent,
@@ -149,12 +208,12 @@ __device__ __forceinline__ void h_sums(int t, const State& st, const unsigned* _
   const unsigned c = min(nbr_cnt[t], cap);
   const unsigned* lst = nbr + nbr_slot((unsigned)t, 0u, cap);
   unsigned jn[kGather], jn2[kGather];
-  list_chunk<kGather>(lst, 0u, c, sent, jn);
-  list_chunk<kGather>(lst, kGather, c, sent, jn2);
+  list_chunk<kGather, 1>(lst, 0u, c, sent, jn);
+  list_chunk<kGather, 1>(lst, kGather, c, sent, jn2);
   for (unsigned k0 = 0; k0 < c; k0 += kGather) {
     float4 pj[kGather];
     float mj[kGather];
-    gather_pos_mass(st, lst, k0, c, sent, jn, jn2, pj, mj);
+    gather_pos_mass<1>(st, lst, k0, c, sent, jn, jn2, pj, mj);
 #pragma unroll
     for (int u = 0; u < kGather; ++u) {
       float ri;
@@ -187,29 +246,40 @@ __device__ __forceinline__ float h_newton(float h, float m, float rho, float drh
   return hn;
 }
 
-template <int KERNEL>
+// One pass of the solve. The new lengths go beside the positions into the state's other buffer (`moved`), which the next
+// pass reads, or, without one, to hnew. The last pass leaves them and gives the density and the residual's maximum.
+template <int KERNEL, int L>
 __global__ void k_h_iter(int n, State st, const unsigned* __restrict__ nbr, const unsigned* __restrict__ nbr_cnt,
                          unsigned cap, unsigned sent, const float* __restrict__ h0, float eta, DevParams* P, Seg* __restrict__ segs,
-                         float* __restrict__ hnew, int last, const Eos* __restrict__ eos, float* __restrict__ rho_out,
-                         float4* __restrict__ fdata) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  float res = 0.0f;
-  const unsigned sg = t < n ? st.seg[t] : kNoSeg;
-  if (t < n) {
-    float rho, drho;
-    h_sums<KERNEL>(t, st, nbr, nbr_cnt, cap, sent, rho, drho);
-    const float m = st.mass[t], h = st.pos_h[t].w;
+                         float* __restrict__ hnew, float4* __restrict__ moved, int last, const Eos* __restrict__ eos,
+                         float* __restrict__ rho_out, float4* __restrict__ fdata) {
+  __shared__ float s[2 * kMaxBlk / L];
+  const int np = blockDim.x / L, first = blockIdx.x * np;
+  const int g = first + (int)threadIdx.x / L, t = first + (int)threadIdx.x;
+  const bool mine = (int)threadIdx.x < np && t < n;
+  float res = 0.0f, rho = 0.0f, drho = 0.0f;
+  const unsigned sg = mine ? st.seg[t] : kNoSeg;
+  if constexpr (L == 1) {
+    if (mine) h_sums<KERNEL>(t, st, nbr, nbr_cnt, cap, sent, rho, drho);
+  } else {
+    block_sums<KERNEL, L>(g < n ? g : -1, mine ? t : -1, st, nbr, nbr_cnt, cap, sent, s, rho, drho);
+  }
+  if (mine) {
+    const float4 p = st.pos_h[t];
+    const float m = st.mass[t];
     float drel;
-    float hn = h_newton(h, m, rho, drho, eta, h0[t], segs[sg].skin, res, drel);
+    const float hn = h_newton(p.w, m, rho, drho, eta, h0[t], segs[sg].skin, res, drel);
     if (last) {
       // the final pass is the density pass: same sum, same order as k_density_eos
       rho_out[t] = rho;
       fdata[t] = eos_record(eos, st.mat[t], m, rho, st.vel_u[t].w, P);
-      hn = h;
+    } else if (moved) {
+      moved[t] = make_float4(p.x, p.y, p.z, hn);
+    } else {
+      hnew[t] = hn;
     }
-    hnew[t] = hn;
   }
-  seg_res_max(segs, sg, res);
+  if (last) seg_res_max(segs, sg, res);
 }
 
 constexpr float kDensityTolFraction = 0.25f;
@@ -282,21 +352,20 @@ __global__ void k_h_commit(int n, State st, const float* __restrict__ hnew) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < n) st.pos_h[t].w = hnew[t];
 }
-__global__ void k_h_reset(DevParams* P, Seg* segs, int nseg, int iters) {
-  if (threadIdx.x < nseg) segs[threadIdx.x].res_bits = 0u;
-  if (threadIdx.x == 0) {
-    P->h_iters_used = (unsigned)iters;
-    P->h_accepted = 0u;
-  }
+__global__ void k_h_reset(DevParams* P, int iters) {
+  P->h_iters_used = (unsigned)iters;
+  P->h_accepted = 0u;
 }
 // The solve's residual maximum (over all impacts); and each impact's next skin: wide while some particle of it
-// is still far from its smoothing length (right after an upload, or a shock), narrow once every one is near it.
-__global__ void k_h_publish(DevParams* P, Seg* segs, int nseg) {
+// is still far from its smoothing length (right after an upload, or a shock), narrow once every one is near it. The
+// maxima are zero again for the next solve. iters >= 0: a full solve's passes (a learned one has set its own figures).
+__global__ void k_h_publish(DevParams* P, Seg* segs, int nseg, int iters) {
   __shared__ float s_max[kMaxSegments / 32];
   float r = 0.0f;
   if (threadIdx.x < nseg) {
     r = __uint_as_float(segs[threadIdx.x].res_bits);
     segs[threadIdx.x].skin = r > P->skin_reset ? P->skin_wide : P->skin_narrow;
+    segs[threadIdx.x].res_bits = 0u;
   }
   r = warp_max(r);
   if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = r;
@@ -305,24 +374,43 @@ __global__ void k_h_publish(DevParams* P, Seg* segs, int nseg) {
     float m = 0.0f;
     for (int k = 0; k < kMaxSegments / 32; ++k) m = fmaxf(m, s_max[k]);
     P->h_residual = m;
+    if (iters >= 0) {
+      P->h_iters_used = (unsigned)iters;
+      P->h_accepted = 0u;
+    }
   }
 }
 
 int launch_h_solve(const Dev& d, const Cfg& c, cudaStream_t s) {
-  const int blocks = (d.n + c.blk - 1) / c.blk;
+  const int lanes = c.learned ? 1 : density_lanes(d.n), blocks = gather_blocks(d.n, c.blk, lanes);
+  const auto pick = [&](auto k) {
+    constexpr int K = decltype(k)::value;
+    return lanes == 4 ? k_h_iter<K, 4> : lanes == 2 ? k_h_iter<K, 2> : k_h_iter<K, 1>;
+  };
+  const auto kernel = c.kernel == 1 ? pick(std::integral_constant<int, 1>{}) : pick(std::integral_constant<int, 0>{});
+  // The passes take turns between the two buffers of positions and lengths, so that the lengths need no commit (3 µs and
+  // a launch each); an odd one out is done first, through hnew, so that the last pass finds them where they belong. Above
+  // 300,000 particles the second buffer costs more than a commit (the step with three contexts at once, in turns and with
+  // commits: 262,144 particles 1,427 and 1,431 µs, 1,048,576 6,270 and 6,200, 1,500,000 9,420 and 8,960).
+  const bool turns = d.n <= 300000;
+  State st = d.s();
+  float4 *here = st.pos_h, *there = d.st[d.cur ^ 1].pos_h;
+  int launches = 0;
   for (int it = 0; it <= c.h_iters; ++it) {
-    const int last = it == c.h_iters;
-    k_h_reset<<<1, kMaxSegments, 0, s>>>(d.P, d.segs, d.nseg, c.h_iters);
-    if (c.kernel == 1)
-      k_h_iter<1><<<blocks, c.blk, 0, s>>>(d.n, d.s(), d.nbr, d.nbr_cnt, d.nbr_cap, d.sent, d.h0, c.h_eta, d.P, d.segs, d.hnew,
-                                          last, d.eos, d.rho, d.fdata);
-    else
-      k_h_iter<0><<<blocks, c.blk, 0, s>>>(d.n, d.s(), d.nbr, d.nbr_cnt, d.nbr_cap, d.sent, d.h0, c.h_eta, d.P, d.segs, d.hnew,
-                                          last, d.eos, d.rho, d.fdata);
-    if (!last) k_h_commit<<<blocks, c.blk, 0, s>>>(d.n, d.s(), d.hnew);
+    const int last = it == c.h_iters, commit = !last && (!turns || (it == 0 && (c.h_iters & 1)));
+    kernel<<<blocks, c.blk, 0, s>>>(d.n, st, d.nbr, d.nbr_cnt, d.nbr_cap, d.sent, d.h0, c.h_eta, d.P, d.segs, d.hnew,
+                                    commit ? nullptr : there, last, d.eos, d.rho, d.fdata);
+    ++launches;
+    if (commit) {
+      k_h_commit<<<(d.n + 255) / 256, 256, 0, s>>>(d.n, st, d.hnew);
+      ++launches;
+    } else {
+      std::swap(here, there);
+      st.pos_h = here;
+    }
   }
-  k_h_publish<<<1, kMaxSegments, 0, s>>>(d.P, d.segs, d.nseg);
-  return (c.h_iters + 1) * 2 + c.h_iters + 1;
+  k_h_publish<<<1, kMaxSegments, 0, s>>>(d.P, d.segs, d.nseg, c.h_iters);
+  return launches + 1;
 }
 
 // Learned h: the proposals written into pos_h.w before the tree build are checked in one pass over all
@@ -331,30 +419,24 @@ int launch_h_solve(const Dev& d, const Cfg& c, cudaStream_t s) {
 int launch_h_learned(const Dev& d, const Cfg& c, cudaStream_t s) {
   const int full = (d.n + c.blk - 1) / c.blk;
   const int part = full < 148 * 8 ? full : 148 * 8;
-  k_h_reset<<<1, kMaxSegments, 0, s>>>(d.P, d.segs, d.nseg, c.h_iters);
+  k_h_reset<<<1, 1, 0, s>>>(d.P, c.h_iters);
   cudaMemsetAsync(d.pend_n, 0, 2 * sizeof(unsigned), s);
   int launches = 2;
-#define HC_ARGS(list, ln, nx, nxn, last)                                                                   \
-  d.n, list, ln, d.s(), d.nbr, d.nbr_cnt, d.nbr_cap, d.sent, d.h0, c.h_eta, c.h_tol, d.P, d.segs, d.hnew, nx, nxn, last, \
-      d.eos, d.rho, d.fdata
-  if (c.kernel == 1)
-    k_h_check<1><<<full, c.blk, 0, s>>>(HC_ARGS(nullptr, nullptr, d.pend[0], d.pend_n, c.h_iters == 0 ? 1 : 0));
-  else
-    k_h_check<0><<<full, c.blk, 0, s>>>(HC_ARGS(nullptr, nullptr, d.pend[0], d.pend_n, c.h_iters == 0 ? 1 : 0));
-  ++launches;
+  const auto check = [&](int blocks, const unsigned* list, const unsigned* list_n, int next, int last) {
+    const auto kernel = c.kernel == 1 ? k_h_check<1> : k_h_check<0>;
+    kernel<<<blocks, c.blk, 0, s>>>(d.n, list, list_n, d.s(), d.nbr, d.nbr_cnt, d.nbr_cap, d.sent, d.h0, c.h_eta, c.h_tol,
+                                    d.P, d.segs, d.hnew, d.pend[next], d.pend_n + next, last, d.eos, d.rho, d.fdata);
+    ++launches;
+  };
+  check(full, nullptr, nullptr, 0, c.h_iters == 0 ? 1 : 0);
   for (int it = 1; it <= c.h_iters; ++it) {
     const int a = (it - 1) & 1, b = it & 1;
     k_h_commit_list<<<part, 256, 0, s>>>(d.pend[a], d.pend_n + a, d.s(), d.hnew);
     cudaMemsetAsync(d.pend_n + b, 0, sizeof(unsigned), s);
-    const int last = it == c.h_iters ? 1 : 0;
-    if (c.kernel == 1)
-      k_h_check<1><<<part, c.blk, 0, s>>>(HC_ARGS(d.pend[a], d.pend_n + a, d.pend[b], d.pend_n + b, last));
-    else
-      k_h_check<0><<<part, c.blk, 0, s>>>(HC_ARGS(d.pend[a], d.pend_n + a, d.pend[b], d.pend_n + b, last));
-    launches += 3;
+    launches += 2;
+    check(part, d.pend[a], d.pend_n + a, b, it == c.h_iters ? 1 : 0);
   }
-#undef HC_ARGS
-  k_h_publish<<<1, kMaxSegments, 0, s>>>(d.P, d.segs, d.nseg);
+  k_h_publish<<<1, kMaxSegments, 0, s>>>(d.P, d.segs, d.nseg, -1);
   return launches + 1;
 }
 
@@ -363,28 +445,36 @@ int launch_h_learned(const Dev& d, const Cfg& c, cudaStream_t s) {
 // :263-269) reduced to each impact's minimum with one atomic per warp (per lane in a warp that straddles two
 // impacts).
 // ---------------------------------------------------------------------------------------------------
-constexpr int kForceGather = 2;  // neighbours of a force chunk (three records each)
+constexpr int kForceGather = 2;  // neighbours of a lane's force chunk (three records each)
 
+constexpr int force_lanes(bool divv) { return divv ? 1 : 4; }
+
+// Four lanes to a particle (10,240 particles 22.5 µs, with a lane to a particle 49; 131,072 99 and 116; 262,144 176 and
+// 192; 1,048,576 644 and 623 by itself, but not with three contexts at once: 5,960 the step, 5,935). With ∇·v, an input
+// of the learned smoothing lengths, one lane sums the list in its order: the network takes it in 16 bits, and another
+// order of the sum moves some inputs by a whole step of those.
 template <int KERNEL, bool GRAV, bool DIVV>
 __global__ void k_forces(int n, State st, const float4* __restrict__ fdata, const unsigned* __restrict__ nbr,
                          const unsigned* __restrict__ nbr_cnt, unsigned cap, unsigned sent,
                          const float4* __restrict__ grav, const DevParams* __restrict__ P, Seg* __restrict__ segs,
                          float4* __restrict__ acc, float* __restrict__ divv) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int L = force_lanes(DIVV);
+  const int t = (blockIdx.x * blockDim.x + threadIdx.x) / L, sub = threadIdx.x & (L - 1);
   float sig = __int_as_float(0x7f800000);
   const unsigned sg = t < n ? st.seg[t] : kNoSeg;
+  float ax = 0.f, ay = 0.f, az = 0.f, de = 0.f, dv = 0.f;
+  float4 pi = make_float4(0.f, 0.f, 0.f, 0.f), vi = pi, fi = pi;
   if (t < n) {
-    const float4 pi = st.pos_h[t];
-    const float4 vi = st.vel_u[t];
-    const float4 fi = fdata[t];
+    pi = st.pos_h[t];
+    vi = st.vel_u[t];
+    fi = fdata[t];
     const float alpha = P->av_alpha, beta = P->av_beta, r_min = P->r_min;
-    float ax = 0.f, ay = 0.f, az = 0.f, de = 0.f, dv = 0.f;
     const unsigned c = min(nbr_cnt[t], cap);
     const unsigned* lst = nbr + nbr_slot((unsigned)t, 0u, cap);
     unsigned jn[kForceGather], jn2[kForceGather];
-    list_chunk<kForceGather>(lst, 0u, c, sent, jn);
-    list_chunk<kForceGather>(lst, kForceGather, c, sent, jn2);
-    for (unsigned k0 = 0; k0 < c; k0 += kForceGather) {
+    list_chunk<kForceGather, L>(lst, (unsigned)sub, c, sent, jn);
+    list_chunk<kForceGather, L>(lst, (unsigned)sub + kForceGather * L, c, sent, jn2);
+    for (unsigned k0 = (unsigned)sub; k0 < c; k0 += kForceGather * L) {
       // a chunk's positions, velocities and force records in flight together, the indices of the two chunks
       // after it requested ahead of them (one chunk ahead left the loads waiting on the list stream)
       unsigned jj[kForceGather];
@@ -394,7 +484,7 @@ __global__ void k_forces(int n, State st, const float4* __restrict__ fdata, cons
         jj[u] = jn[u];
         jn[u] = jn2[u];
       }
-      list_chunk<kForceGather>(lst, k0 + 2 * kForceGather, c, sent, jn2);
+      list_chunk<kForceGather, L>(lst, k0 + 2 * kForceGather * L, c, sent, jn2);
 #pragma unroll
       for (int u = 0; u < kForceGather; ++u) {
         pjs[u] = st.pos_h[jj[u]];
@@ -434,6 +524,14 @@ __global__ void k_forces(int n, State st, const float4* __restrict__ fdata, cons
         if (DIVV) dv += fj.x * vg;
       }
     }
+  }
+  if constexpr (L > 1) {
+    ax = add_shares<L>(&ax);
+    ay = add_shares<L>(&ay);
+    az = add_shares<L>(&az);
+    de = add_shares<L>(&de);
+  }
+  if (t < n && sub == 0) {
     if (GRAV) {
       const float4 g = grav[t];
       ax += g.x;
@@ -457,25 +555,16 @@ __global__ void k_forces(int n, State st, const float4* __restrict__ fdata, cons
 }
 
 int launch_forces(const Dev& d, const Cfg& c, cudaStream_t s) {
-  const int blocks = (d.n + c.blk - 1) / c.blk;
   const bool g = c.gravity != 2;
-#define FARGS d.n, d.s(), d.fdata, d.nbr, d.nbr_cnt, d.nbr_cap, d.sent, d.grav, d.P, d.segs, d.acc, d.divv
-  if (c.divv) {
-    if (c.kernel == 1) {
-      if (g) k_forces<1, true, true><<<blocks, c.blk, 0, s>>>(FARGS);
-      else k_forces<1, false, true><<<blocks, c.blk, 0, s>>>(FARGS);
-    } else {
-      if (g) k_forces<0, true, true><<<blocks, c.blk, 0, s>>>(FARGS);
-      else k_forces<0, false, true><<<blocks, c.blk, 0, s>>>(FARGS);
-    }
-  } else if (c.kernel == 1) {
-    if (g) k_forces<1, true, false><<<blocks, c.blk, 0, s>>>(FARGS);
-    else k_forces<1, false, false><<<blocks, c.blk, 0, s>>>(FARGS);
-  } else {
-    if (g) k_forces<0, true, false><<<blocks, c.blk, 0, s>>>(FARGS);
-    else k_forces<0, false, false><<<blocks, c.blk, 0, s>>>(FARGS);
-  }
-#undef FARGS
+  const auto by_divv = [&](auto k, auto gr) {
+    constexpr int K = decltype(k)::value;
+    constexpr bool G = decltype(gr)::value;
+    return c.divv ? k_forces<K, G, true> : k_forces<K, G, false>;
+  };
+  const auto pick = [&](auto k) { return g ? by_divv(k, std::true_type{}) : by_divv(k, std::false_type{}); };
+  const auto kernel = c.kernel == 1 ? pick(std::integral_constant<int, 1>{}) : pick(std::integral_constant<int, 0>{});
+  kernel<<<gather_blocks(d.n, c.blk, force_lanes(c.divv)), c.blk, 0, s>>>(
+      d.n, d.s(), d.fdata, d.nbr, d.nbr_cnt, d.nbr_cap, d.sent, d.grav, d.P, d.segs, d.acc, d.divv);
   return 1;
 }
 
