@@ -684,14 +684,15 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
   };
   // Rounds of F chunks, one for each warp; a particle's list takes the warps' finds in their order, so the list is
   // that of a single warp going through the chunks.
+  constexpr unsigned kBatch = 4;
   const bool one_by_one = HILO || (GRAV && soft2 < kNearSoft2);
   auto flush_p2p = [&](int count) {
     const int per = near_per;  // leaves per chunk
     float4 nsrc;
     float nh;
     int nidx = near_source(w * per, count, nsrc, nh);
-    unsigned turn = 0u;
-    for (int base = 0; base < count; base += per * F, turn ^= 1u) {
+    unsigned turn = 0u, finds = 0u;
+    for (int base = 0; base < count; base += per * F) {
       const int mine = base + w * per;
       float4 src = nsrc;
       const float hsrc = nh;
@@ -702,7 +703,7 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
         part_src += __popc(__ballot_sync(SPH_FULL_MASK, sidx >= 0));
         nidx = near_source(mine + per * F, count, nsrc, nh);
         src.w *= G;
-        S.idx[w][lane] = sidx;
+        if (F > 1 || one_by_one) S.idx[w][lane] = sidx;
         if (NBR) S.hs[w][lane] = hsrc;
         if (one_by_one) {
           S.src[w][lane] = src;
@@ -742,25 +743,49 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
           }
         }
       }
-      if (NBR) {
-        unsigned at = cnt;
-        if constexpr (F == 1) {
-          cnt += (unsigned)__popc(found);
-        } else {
-          S.hits[turn][w][lane] = (unsigned)__popc(found);
-          __syncthreads();
-#pragma unroll
-          for (int k = 0; k < F; ++k) {
-            const unsigned h = S.hits[turn][k][lane];
-            at += k < w ? h : 0u;
-            cnt += h;
+      if constexpr (NBR && F == 1) {
+        // A batch of kBatch chunks' finds is written at once: a lane goes from chunk to chunk by itself, and the warp waits
+        // for the longest sum of a batch, not for the sum of every chunk's longest.
+        unsigned* masks = reinterpret_cast<unsigned*>(&S.q0[w][0]);
+        masks[32 * turn + lane] = found;
+        finds += (unsigned)__popc(found);
+        if (++turn == kBatch || base + per >= count) {
+          unsigned left = min(finds, cap - min(cnt, cap));
+          unsigned* out = nlst + (size_t)cnt * 32u;
+          cnt += finds;
+          const unsigned* e = S.p2p + (base - ((int)turn - 1) * per);  // the chunk's leaves
+          const unsigned* row = masks + lane;
+          unsigned m = *row;
+          for (; left; --left, out += 32) {
+            while (!m) {
+              row += 32;
+              e += per;
+              m = *row;
+            }
+            const int k = __clz(m);
+            m &= ~(0x80000000u >> k);
+            *out = (e[k >> ksh] >> 5) + (unsigned)(k & (K - 1));
           }
+          finds = 0u;
+          turn = 0u;
+        }
+      }
+      if constexpr (NBR && F > 1) {
+        unsigned at = cnt;
+        S.hits[turn][w][lane] = (unsigned)__popc(found);
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < F; ++k) {
+          const unsigned h = S.hits[turn][k][lane];
+          at += k < w ? h : 0u;
+          cnt += h;
         }
         for (; found; ++at) {
           const int k = __clz(found);
           found &= ~(0x80000000u >> k);
           if (at < cap) nlst[(size_t)at * 32u] = (unsigned)S.idx[w][k];
         }
+        turn ^= 1u;
       }
       __syncwarp();
     }
