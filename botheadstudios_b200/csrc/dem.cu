@@ -150,8 +150,12 @@ __global__ void k_dem_contacts(int n, State st, const unsigned* __restrict__ nbr
   // Only gaps below the 1 cm projection cap matter, and those grains are all contact candidates.
   const bool terrain = p.hf != nullptr;
   const float3 tn = terrain ? terrain_normal(terrain_surface(p, pi.x, pi.z)) : make_float3(0.f, 1.f, 0.f);
+  const uint4* row = reinterpret_cast<const uint4*>(nbr + nbr_slot((unsigned)t, 0u, cap));  // four entries, 32 apart
+  uint4 four = make_uint4(0u, 0u, 0u, 0u);
   for (unsigned k = 0; k < c; ++k) {
-    const unsigned j = nbr[nbr_slot((unsigned)t, k, cap)];
+    if ((k & 3u) == 0u) four = row[(size_t)(k >> 2) * 32u];
+    const unsigned j = four.x;
+    four = make_uint4(four.y, four.z, four.w, 0u);
     const float4 pj = st.pos_h[j];
     const float rj = st.mass[j];
     dem_pair(pi, vi, ri, pj, st.vel_u[j], rj, p, f, sd, so, sv);

@@ -38,7 +38,7 @@ __device__ __forceinline__ float pair_h(float hi, float hj) { return fmul(0.5f, 
 // A lane takes G of its entries at a time: all of a chunk's indices are loaded, then all of its neighbour records,
 // before any is used, so it keeps G gathers in flight instead of one dependent chain; the indices are requested two
 // chunks ahead of the records, so the list stream (HBM) overlaps the record gathers (mostly L1/L2) and the arithmetic.
-// `lst` is the particle's first list slot (entries 32 apart, interleaved); slots past the count read the sentinel record
+// `lst` is the particle's first list slot (nbr_slot); slots past the count read the sentinel record
 // `sent` (a massless particle outside every support), so a pair is evaluated without testing the count or the support
 // (kern_pair_bf vanishes outside it). The lists are read once per pass and streamed past the cache (evict-first), so
 // they do not push the neighbours' records out of L2.
@@ -47,8 +47,23 @@ constexpr int kGather = 4;
 template <int G, int L>
 __device__ __forceinline__ void list_chunk(const unsigned* __restrict__ lst, unsigned k0, unsigned c, unsigned sent,
                                            unsigned j[G]) {
+  const unsigned* at = lst + (size_t)(k0 & ~3u) * 32u + (k0 & 3u);
+  if constexpr (L == 1) {  // (k0 a multiple of G)
+    if constexpr (G == 4) {
+      const uint4 v = k0 < c ? __ldcs(reinterpret_cast<const uint4*>(at)) : make_uint4(0u, 0u, 0u, 0u);
+      j[0] = v.x, j[1] = v.y, j[2] = v.z, j[3] = v.w;
+    } else {
+      static_assert(G == 2, "a chunk is half a row's entries or all of them");
+      const uint2 v = k0 < c ? __ldcs(reinterpret_cast<const uint2*>(at)) : make_uint2(0u, 0u);
+      j[0] = v.x, j[1] = v.y;
+    }
 #pragma unroll
-  for (int u = 0; u < G; ++u) j[u] = k0 + u * L < c ? __ldcs(&lst[(size_t)(k0 + u * L) * 32u]) : sent;
+    for (int u = 0; u < G; ++u) j[u] = k0 + u < c ? j[u] : sent;
+  } else {  // (k0 the lane's place in a row and a multiple of four)
+#pragma unroll
+    for (int u = 0; u < G; ++u)
+      j[u] = k0 + u * L < c ? __ldcs(at + (L == 4 ? 128 * u : 128 * (u >> 1) + 2 * (u & 1))) : sent;
+  }
 }
 // Records of the chunk whose indices are in `jn` (k0 = its first slot); jn2 holds the next chunk's indices.
 // On return jn holds the next chunk's and jn2 the one after it: the list stays two chunks ahead of the records.

@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
   };
   // The sources of a chunk that passed the neighbour test, one bit each (the first source's bit highest).
   unsigned found = 0u;
-  // (the particle's first list slot once, entries 32 apart: the interleaved layout of nbr_slot)
+  // (the particle's first list slot once: the interleaved layout of nbr_slot)
   unsigned* const nlst = NBR ? nbr + nbr_slot((unsigned)t, 0u, cap) : nullptr;
   // Sources in pairs, as in the far loop (their smoothing lengths in hs); every packed operation rounds as its scalar
   // form, so the distances and the predicate are those of the scalar loop below, source by source. A test is the sign
@@ -751,12 +751,12 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
         finds += (unsigned)__popc(found);
         if (++turn == kBatch || base + per >= count) {
           unsigned left = min(finds, cap - min(cnt, cap));
-          unsigned* out = nlst + (size_t)cnt * 32u;
+          unsigned* out = nlst + (size_t)(cnt & ~3u) * 32u + (cnt & 3u);
           cnt += finds;
           const unsigned* e = S.p2p + (base - ((int)turn - 1) * per);  // the chunk's leaves
           const unsigned* row = masks + lane;
           unsigned m = *row;
-          for (; left; --left, out += 32) {
+          for (; left; --left) {
             while (!m) {
               row += 32;
               e += per;
@@ -765,6 +765,8 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
             const int k = __clz(m);
             m &= ~(0x80000000u >> k);
             *out = (e[k >> ksh] >> 5) + (unsigned)(k & (K - 1));
+            // the next entry of the row, or the next row's first
+            out += (reinterpret_cast<uintptr_t>(out) & 12u) == 12u ? 125 : 1;
           }
           finds = 0u;
           turn = 0u;
@@ -783,7 +785,7 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
         for (; found; ++at) {
           const int k = __clz(found);
           found &= ~(0x80000000u >> k);
-          if (at < cap) nlst[(size_t)at * 32u] = (unsigned)S.idx[w][k];
+          if (at < cap) nlst[(size_t)(at & ~3u) * 32u + (at & 3u)] = (unsigned)S.idx[w][k];
         }
         turn ^= 1u;
       }

@@ -147,7 +147,7 @@ sph_status alloc_dev(sph_ctx* ctx, Dev& d, uint32_t cap, uint32_t K, uint32_t nb
   ALLOC(d.P, 1);
   if (sph) {
     d.nbr_cap = nbr_cap;
-    ALLOC(d.nbr, capw * nbr_cap);
+    ALLOC(d.nbr, capw * 4 * nbr_rows(nbr_cap));
     ALLOC(d.nbr_cnt, capw);
     ALLOC(d.rho, capw);
     ALLOC(d.fdata, capw + 32);
@@ -1074,7 +1074,7 @@ sph_status sph_inspect(sph_ctx* ctx, uint32_t what, void* host_out, size_t bytes
       const size_t cap = d.nbr_cap;
       if (!need(n * cap * 4)) return SPH_ERR_INVALID;
       const size_t groups = (n + 31) / 32;
-      std::vector<unsigned> lst(groups * cap * 32), cnt(n);
+      std::vector<unsigned> lst(groups * nbr_rows((unsigned)cap) * 128), cnt(n);
       CK(cudaMemcpy(lst.data(), d.nbr, lst.size() * 4, cudaMemcpyDeviceToHost));
       CK(cudaMemcpy(cnt.data(), d.nbr_cnt, n * 4, cudaMemcpyDeviceToHost));
       sph_status st = load_ids();
@@ -1083,7 +1083,7 @@ sph_status sph_inspect(sph_ctx* ctx, uint32_t what, void* host_out, size_t bytes
       std::memset(o, 0xff, n * cap * 4);
       for (size_t t = 0; t < n; ++t) {
         const size_t c = cnt[t] < cap ? cnt[t] : cap;
-        for (size_t k = 0; k < c; ++k) o[ids[t] * cap + k] = ids[lst[((t >> 5) * cap + k) * 32 + (t & 31)]];
+        for (size_t k = 0; k < c; ++k) o[ids[t] * cap + k] = ids[lst[nbr_slot((unsigned)t, (unsigned)k, (unsigned)cap)]];
       }
       return SPH_OK;
     }

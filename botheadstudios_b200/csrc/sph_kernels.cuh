@@ -166,7 +166,7 @@ struct Dev {
   uint2* groups = nullptr;      // [L] walk groups: (first leaf, last leaf) of runs of 32/K leaves of one impact
   int ngroups = 0;              // number of groups
   int shared_groups = 0;        // ... of which the first are walked by several warps each (kSharedWalkMax)
-  unsigned* nbr = nullptr;      // interleaved neighbour lists [n/32][nbr_cap][32]
+  unsigned* nbr = nullptr;      // interleaved neighbour lists [n/32][nbr_rows(nbr_cap)][32][4]
   unsigned* nbr_cnt = nullptr;  // [n]
   unsigned nbr_cap = 0;
   float* rho = nullptr;         // [n]
