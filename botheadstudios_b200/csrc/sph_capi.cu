@@ -1503,7 +1503,7 @@ sph_status sph_dem_step(sph_dem* dem, uint32_t substeps) {
   Dev& d = ctx->d;
   cudaStream_t s = ctx->stream;
   for (uint32_t k = 0; k < substeps; ++k) {
-    phase(ctx, SPH_PHASE_SORT, [&] { return launch_sort_permute(d, true, s); });
+    phase(ctx, SPH_PHASE_SORT, [&] { return launch_sort_permute(d, !dem->stepped && k == 0, s); });
     phase(ctx, SPH_PHASE_TREE, [&] { return launch_tree(d, ctx->kc, ctx->cfg.theta, s); });
     phase(ctx, SPH_PHASE_NEIGHBOURS, [&] { return launch_neighbours(d, ctx->kc, s); });
     phase(ctx, SPH_PHASE_FORCES, [&] { return launch_dem_contacts(d, dem->p, dem->acc, s); });
