@@ -49,26 +49,7 @@ int launch_segments(const Dev& d, cudaStream_t s) {
 }
 
 __global__ void k_segments_single(Seg* segs, int n, int L, float soft2, double dt) {
-  Seg a;
-  a.off = 0u;
-  a.loff = 0u;
-  a.root = 0u;
-  a.sig_bits = 0x7f800000u;
-  for (int k = 0; k < 3; ++k) {
-    a.bbox[k] = 0xffffffffu;
-    a.bbox[3 + k] = 0u;
-  }
-  a.soft2 = soft2;
-  a.pad = 0u;
-  a.res_bits = 0u;
-  a.skin = 0.0f;
-  a.dt = dt;
-  a.time = 0.0;
-  segs[0] = a;
-  Seg e = a;
-  e.off = (unsigned)n;
-  e.loff = (unsigned)L;
-  segs[1] = e;
+  write_single_segment(segs, n, L, soft2, dt);
 }
 
 int launch_segments_single(const Dev& d, float soft2, double dt, cudaStream_t s) {

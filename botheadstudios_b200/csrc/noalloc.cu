@@ -186,29 +186,38 @@ Dev carve_dev(unsigned char* base, uint32_t K) {
   return d;
 }
 
-// Everything the walk reads from DevParams, written on the device (no host copy), counters cleared.
-__global__ void k_noalloc_params(DevParams* P, float G, float theta) {
+// Everything the walk reads from DevParams, written on the device (no host copy), counters cleared; the segment table.
+__global__ void k_noalloc_params(DevParams* P, Seg* segs, int n, int L, float soft2, float G, float theta) {
   DevParams p;
   memset(&p, 0, sizeof(p));
   p.G = G;
   p.theta = theta;
   *P = p;
+  write_single_segment(segs, n, L, soft2, 0.0);
 }
 
-__global__ void k_noalloc_load(const float4* __restrict__ in, int n, State st) {
+// The points and their bounding box (three launches fewer than with a reset, a box and a segment kernel of their own:
+// 16,001 points 263 µs instead of 273).
+__global__ void __launch_bounds__(256) k_noalloc_load(const float4* __restrict__ in, int n, State st, Seg* segs) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float4 b = in[i];
-  st.pos_h[i] = make_float4(b.x, b.y, b.z, 0.0f);
-  st.vel_u[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  st.x[i] = (double)b.x;
-  st.y[i] = (double)b.y;
-  st.z[i] = (double)b.z;
-  st.mass[i] = b.w;
-  st.mat[i] = 0u;
-  st.prov[i] = 0u;
-  st.id[i] = (unsigned)i;
-  st.seg[i] = 0u;
+  unsigned lo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, hi[3] = {0u, 0u, 0u};
+  if (i < n) {
+    const float4 b = in[i];
+    st.pos_h[i] = make_float4(b.x, b.y, b.z, 0.0f);
+    st.vel_u[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    st.x[i] = (double)b.x;
+    st.y[i] = (double)b.y;
+    st.z[i] = (double)b.z;
+    st.mass[i] = b.w;
+    st.mat[i] = 0u;
+    st.prov[i] = 0u;
+    st.id[i] = (unsigned)i;
+    st.seg[i] = 0u;
+    lo[0] = hi[0] = float_key(b.x);
+    lo[1] = hi[1] = float_key(b.y);
+    lo[2] = hi[2] = float_key(b.z);
+  }
+  seg_bbox_commit(lo, hi, i < n ? 0u : kNoSeg, segs);
 }
 
 // The results in input order. If the walk's traversal stack overflowed (it then skips subtrees), every
@@ -253,10 +262,10 @@ extern "C" sph_status sph_gravity_tree_noalloc(const void* d_bodies4, uint32_t n
   c.quad = (int)multipole;
   c.mac = SPH_MAC_GROUP;
   c.local_theta = kLocalThetaDefault;  // the walk sph_gravity runs with the default configuration
-  k_noalloc_params<<<1, 1, 0, s>>>(d.P, (float)G, theta);
-  k_noalloc_load<<<(n + 255) / 256, 256, 0, s>>>(static_cast<const float4*>(d_bodies4), (int)n, d.st[0]);
-  launch_segments_single(d, softening * softening, 0.0, s);
-  launch_sort_permute(d, true, s);
+  k_noalloc_params<<<1, 1, 0, s>>>(d.P, d.segs, d.n, d.L, softening * softening, (float)G, theta);
+  k_noalloc_load<<<(n + 255) / 256, 256, 0, s>>>(static_cast<const float4*>(d_bodies4), (int)n, d.st[0], d.segs);
+  launch_segments(d, s);
+  launch_sort_permute(d, false, s);
   launch_tree(d, c, theta, s);
   launch_gravity_points(d, c, s);
   k_noalloc_store<<<(n + 255) / 256, 256, 0, s>>>((int)n, d.s().id, d.grav, d.P, static_cast<float4*>(d_acc4));

@@ -56,6 +56,30 @@ struct Seg {
 static_assert(sizeof(Seg) == 72, "Seg is one 72-byte record");
 constexpr unsigned kNoSeg = 0xffffffffu;
 
+// The table of a single impact: an empty bounding box, no simulated time.
+__device__ __forceinline__ void write_single_segment(Seg* segs, int n, int L, float soft2, double dt) {
+  Seg a;
+  a.off = 0u;
+  a.loff = 0u;
+  a.root = 0u;
+  a.sig_bits = 0x7f800000u;
+  for (int k = 0; k < 3; ++k) {
+    a.bbox[k] = 0xffffffffu;
+    a.bbox[3 + k] = 0u;
+  }
+  a.soft2 = soft2;
+  a.pad = 0u;
+  a.res_bits = 0u;
+  a.skin = 0.0f;
+  a.dt = dt;
+  a.time = 0.0;
+  segs[0] = a;
+  Seg e = a;
+  e.off = (unsigned)n;
+  e.loff = (unsigned)L;
+  segs[1] = e;
+}
+
 // Reduce per-thread boxes (order-preserving keys, identity values when the thread holds no point) into the
 // segment table. Particles are contiguous per segment, so almost every block lies in one segment and commits
 // with one atomic per axis; a block that straddles segments commits per warp (warps inside one segment) or
