@@ -202,7 +202,7 @@ __global__ void k_dm_moments_final(const double* __restrict__ part, int nb, doub
 // down from a bound on the radii), a second one in the 4,096 bins of its next 12 bits inside the bin where the running
 // weight crosses, a third lists the points of the crossing bin there, some ten of a million, and one block ranks those.
 // Weights are integers, so the sums do not depend on their order and equal masses sum exactly. Bound by three readings of the points; a radix sort of the 64-bit radii, the masses
-// gathered in its order and two prefixes took 226 µs at 1,024,845 points, the three passes take 52.
+// gathered in its order and two prefixes took 226 µs at 1,024,845 points, the three passes take 50.
 __device__ __forceinline__ unsigned long long radius_bits(float4 p, const double* __restrict__ centre) {
   const double dx = __dsub_rn((double)p.x, centre[0]), dy = __dsub_rn((double)p.y, centre[1]),
                dz = __dsub_rn((double)p.z, centre[2]);
@@ -339,6 +339,7 @@ __global__ void __launch_bounds__(kDmThreads) k_dm_select_radius(const float4* _
                                                                  RadiusSelect* sel, unsigned long long* list_key,
                                                                  unsigned* list_idx, double* __restrict__ out) {
   __shared__ unsigned long long h[kSelBins];
+  unsigned* h32 = reinterpret_cast<unsigned*>(h);  // pass 0: low words, then high words (64-bit shared adds are loops: 25.4 µs, this 23.6)
   __shared__ int s_last;
   const double M = *total_mass, scale = sel_scale(M);
   // the centre is a mean of the points, so no radius is above 2 sqrt(3) times their largest coordinate
@@ -357,7 +358,12 @@ __global__ void __launch_bounds__(kDmThreads) k_dm_select_radius(const float4* _
       const float4 p = pm[i];
       const unsigned long long key = radius_bits(p, centre);
       keys[i] = key;
-      atomicAdd(&h[sel_bin(key, bound)], sel_weight(p.w, scale));
+      const unsigned d = sel_bin(key, bound);
+      const unsigned long long wt = sel_weight(p.w, scale);
+      const unsigned lo = (unsigned)wt;
+      const unsigned carry = atomicAdd(&h32[d], lo) > ~lo ? 1u : 0u;
+      const unsigned up = (unsigned)(wt >> 32) + carry;
+      if (up) atomicAdd(&h32[kSelBins + d], up);
     } else {
       const unsigned long long key = keys[i];
       if (sel_bin(key, bound) == a) {
@@ -375,7 +381,8 @@ __global__ void __launch_bounds__(kDmThreads) k_dm_select_radius(const float4* _
   if (PASS == 0) {
     __syncthreads();
     for (int k = threadIdx.x; k < kSelBins; k += kDmThreads)
-      if (h[k]) atomicAdd(&sel->hist[0][k], h[k]);
+      if (h32[k] | h32[kSelBins + k])
+        atomicAdd(&sel->hist[0][k], (unsigned long long)h32[kSelBins + k] << 32 | h32[k]);
   }
   __threadfence();
   __syncthreads();
@@ -704,59 +711,79 @@ __global__ void k_dm_clumps(unsigned n, const unsigned long long* __restrict__ s
   clump[c] = make_uint4(i, s, order[i], 0u);  // (the sort is stable: the group's smallest index)
 }
 
-// One block per clump: mass, centre of mass, volume, target mass, then the internal kinetic energy.
-__global__ void __launch_bounds__(kDmThreads) k_dm_clump_stats(const unsigned* __restrict__ cnt,
-                                                               const uint4* __restrict__ clump, int variant,
-                                                               const float4* __restrict__ dpos,
-                                                               const float4* __restrict__ dvel,
-                                                               const float2* __restrict__ drp,
-                                                               double* __restrict__ cstat) {
-  __shared__ double s[kDmThreads / 32][kDmVals];
-  __shared__ double s_cv[3];
+// A clump's mass, centre of mass, volume and target mass, then its internal kinetic energy, by `threads` threads of which
+// this is the rank-th; sum() adds eight values over them and gives every thread the result (the order is fixed).
+template <class Sum>
+__device__ __forceinline__ void clump_stats(uint4 cl, unsigned rank, unsigned threads, int variant,
+                                            const float4* __restrict__ dpos, const float4* __restrict__ dvel,
+                                            const float2* __restrict__ drp, double* __restrict__ o, Sum sum) {
+  double a[kDmVals] = {0, 0, 0, 0, 0, 0, 0, 0}, target = 0.0;
+#pragma unroll 4
+  for (unsigned j = rank; j < cl.y; j += threads) {
+    const unsigned t = cl.x + j;
+    const float4 p = dpos[t], v = dvel[t];
+    const float2 rp = drp[t];
+    const double mm = v.w;
+    a[0] += mm;
+    a[1] += (double)v.x * mm;
+    a[2] += (double)v.y * mm;
+    a[3] += (double)v.z * mm;
+    a[4] += (double)p.x * mm;
+    a[5] += (double)p.y * mm;
+    a[6] += (double)p.z * mm;
+    const double rho = variant == 0 ? (double)rp.x : (double)fmaxf(rp.x, 1.0f);  // gpu_sph.rs:450
+    a[7] += mm / rho;
+    target += __float_as_uint(rp.y) == 0u ? mm : 0.0;
+  }
+  sum(a);
+  const double cvx = a[1] / a[0], cvy = a[2] / a[0], cvz = a[3] / a[0];
+  double b[kDmVals] = {0, target, 0, 0, 0, 0, 0, 0};
+#pragma unroll 4
+  for (unsigned j = rank; j < cl.y; j += threads) {
+    const float4 v = dvel[cl.x + j];
+    b[0] += 0.5 * (double)v.w * dsq3((double)v.x - cvx, (double)v.y - cvy, (double)v.z - cvz);
+  }
+  sum(b);
+  if (rank == 0) {
+    o[0] = a[0];
+    o[1] = a[4] / a[0];
+    o[2] = a[5] / a[0];
+    o[3] = a[6] / a[0];
+    o[4] = a[7];
+    o[5] = b[1];
+    o[6] = b[0];
+  }
+}
+
+// Most clumps have a few members and one has most of the disk: a block of 1,024 threads for each of the larger ones, then
+// a warp for each of the rest (a block of 256 for every clump took 37 µs for a disk of 22,840 particles, this 24).
+constexpr unsigned kWarpClump = 128;
+__global__ void __launch_bounds__(1024) k_dm_clump_stats(const unsigned* __restrict__ cnt,
+                                                         const uint4* __restrict__ clump, int variant,
+                                                         const float4* __restrict__ dpos,
+                                                         const float4* __restrict__ dvel,
+                                                         const float2* __restrict__ drp, double* __restrict__ cstat) {
+  __shared__ double s[32][kDmVals], s_total[kDmVals];
   const unsigned ncl = cnt[C_NCLUMP];
   for (unsigned c = blockIdx.x; c < ncl; c += gridDim.x) {
     const uint4 cl = clump[c];
-    double a[kDmVals] = {0, 0, 0, 0, 0, 0, 0, 0}, target = 0.0;
-#pragma unroll 4
-    for (unsigned j = threadIdx.x; j < cl.y; j += kDmThreads) {
-      const unsigned t = cl.x + j;
-      const float4 p = dpos[t], v = dvel[t];
-      const float2 rp = drp[t];
-      const double mm = v.w;
-      a[0] += mm;
-      a[1] += (double)v.x * mm;
-      a[2] += (double)v.y * mm;
-      a[3] += (double)v.z * mm;
-      a[4] += (double)p.x * mm;
-      a[5] += (double)p.y * mm;
-      a[6] += (double)p.z * mm;
-      const double rho = variant == 0 ? (double)rp.x : (double)fmaxf(rp.x, 1.0f);  // gpu_sph.rs:450
-      a[7] += mm / rho;
-      target += __float_as_uint(rp.y) == 0u ? mm : 0.0;
-    }
-    block_sum(a, s);
-    if (threadIdx.x == 0) {
-      for (int k = 0; k < 3; ++k) s_cv[k] = a[1 + k] / a[0];
-      double* o = cstat + (size_t)c * 8;
-      o[0] = a[0];
-      o[1] = a[4] / a[0];
-      o[2] = a[5] / a[0];
-      o[3] = a[6] / a[0];
-      o[4] = a[7];
-    }
-    __syncthreads();
-    double k3[kDmVals] = {0, target, 0, 0, 0, 0, 0, 0};
-    const double cvx = s_cv[0], cvy = s_cv[1], cvz = s_cv[2];
-#pragma unroll 4
-    for (unsigned j = threadIdx.x; j < cl.y; j += kDmThreads) {
-      const float4 v = dvel[cl.x + j];
-      k3[0] += 0.5 * (double)v.w * dsq3((double)v.x - cvx, (double)v.y - cvy, (double)v.z - cvz);
-    }
-    block_sum(k3, s);
-    if (threadIdx.x == 0) {
-      cstat[(size_t)c * 8 + 5] = k3[1];
-      cstat[(size_t)c * 8 + 6] = k3[0];
-    }
+    if (cl.y <= kWarpClump) continue;
+    clump_stats(cl, threadIdx.x, blockDim.x, variant, dpos, dvel, drp, cstat + (size_t)c * 8, [&](double* v) {
+      block_sum(v, s);
+      if (threadIdx.x == 0)
+        for (int k = 0; k < kDmVals; ++k) s_total[k] = v[k];
+      __syncthreads();
+      for (int k = 0; k < kDmVals; ++k) v[k] = s_total[k];
+      __syncthreads();
+    });
+  }
+  const unsigned warps = gridDim.x * (blockDim.x >> 5);
+  for (unsigned c = blockIdx.x + gridDim.x * (threadIdx.x >> 5); c < ncl; c += warps) {
+    const uint4 cl = clump[c];
+    if (cl.y > kWarpClump) continue;
+    clump_stats(cl, threadIdx.x & 31u, 32u, variant, dpos, dvel, drp, cstat + (size_t)c * 8, [](double* v) {
+      for (int k = 0; k < kDmVals; ++k) v[k] = warp_sum(v[k]);
+    });
   }
 }
 
@@ -1259,8 +1286,8 @@ int disk_measure(const Dev& d, unsigned off, unsigned m, const DiskCfg& c, DiskW
                                    w->drp[0], nullptr, nullptr);
     k_dm_clumps<<<gb, 256, 0, s>>>(nd, w->keys[src], w->vals[src], w->gcnt, w->clump, w->cnt);
     const unsigned cb = nd / 2 < 1184u ? nd / 2 : 1184u;  // clumps <= nd / 2; blocks stride over them
-    k_dm_clump_stats<<<cb, kDmThreads, 0, s>>>(w->cnt, w->clump, c.variant, w->dpos[0], w->dvel[0], w->drp[0],
-                                               w->cstat);
+    const unsigned sb = nd / 2 < 296u ? nd / 2 : 296u;  // two blocks of 1,024 threads per SM
+    k_dm_clump_stats<<<sb, 1024, 0, s>>>(w->cnt, w->clump, c.variant, w->dpos[0], w->dvel[0], w->drp[0], w->cstat);
     k_dm_unit_scan<<<1, 1024, 0, s>>>(w->cnt, w->clump, w->uoff);
     L += 4;
     // the self-potential's unit count sizes its partial sums: read it back once
