@@ -4,9 +4,9 @@ A batch of impacts of uneven size is split into size buckets, each tuned on its 
 configurations agree share one context, which advances all of their impacts with one launch per phase (with one
 configuration for every bucket, the whole batch is one context), and contexts of different configurations run
 concurrently on their own streams. The autotuner picks, per bucket, the LBVH leaf size, the block size of the
-per-particle gather kernels (density, h-solve, forces) and the traversal tile of the fused walk (warps per
-block) by timing candidates on a probe batch drawn from that bucket. Choices are cached in a JSON file keyed
-by the GPU name and the bucket.
+per-particle gather kernels (density, h-solve, forces) and the walk's tile (without effect: the walk chooses how
+many warps share a group by the impact's size) by timing candidates on a probe batch drawn from that bucket.
+Choices are cached in a JSON file keyed by the GPU name and the bucket.
 
 The reference has no counterpart: its offline driver runs impacts one after another
 (tools/impact-run/src/main.rs:645-671).

@@ -14,7 +14,7 @@
 // opened the node. Neighbouring points open nearly the same nodes, so a node costs one staging and one test for
 // 32 points, where a walk for each point alone (a warp whose 32 points are 32 groups of one) repeats both 32 times:
 // 16,001 points in 16-point leaves with quadrupoles: a call took 3,394 µs that way (3,305 µs of them in the walk) and
-// takes 346 µs. Bound by latency below about 20,000 points (rounds of dependent loads, hence 8 warps for 32 points)
+// takes 265 µs (202 in the walk). Bound by latency below about 20,000 points (rounds of dependent loads, hence 8 warps for 32 points)
 // and by issue above.
 #include "sph_kernels.cuh"
 

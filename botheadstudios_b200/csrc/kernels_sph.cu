@@ -173,10 +173,10 @@ __global__ void k_density_eos(int n, State st, const unsigned* __restrict__ nbr,
   fdata[t] = eos_record(eos, st.mat[t], st.mass[t], r_i, st.vel_u[t].w, P);
 }
 
-// Lanes a particle takes in the density sums. The density of 10,240 particles 10.7 µs with four lanes, 12.8 with two
-// (14.0 with one); a solve of two passes and the density 61 and 59 (62) at 32,768, 145 and 135 (142) at 180,000, 656 and
-// 562 (512) at 1,048,576 by itself, but with three contexts at once the step there is shorter with two than with one
-// (5,895 and 5,960).
+// Lanes a particle takes in the density sums (measured while a list's entries lay in rows of one). The density of 10,240
+// particles 10.7 µs with four lanes, 12.8 with two (14.0 with one); a solve of two passes and the density 61 and 59 (62)
+// at 32,768, 145 and 135 (142) at 180,000, 656 and 562 (512) at 1,048,576 by itself, but with three contexts at once the
+// step there is shorter with two than with one (5,895 and 5,960).
 static int density_lanes(int n) { return n <= 20000 ? 4 : 2; }
 static int gather_blocks(int n, int blk, int lanes) { return (n + blk / lanes - 1) / (blk / lanes); }
 
@@ -464,10 +464,10 @@ constexpr int kForceGather = 2;  // neighbours of a lane's force chunk (three re
 
 constexpr int force_lanes(bool divv) { return divv ? 1 : 4; }
 
-// Four lanes to a particle (10,240 particles 22.5 µs, with a lane to a particle 49; 131,072 99 and 116; 262,144 176 and
-// 192; 1,048,576 644 and 623 by itself, but not with three contexts at once: 5,960 the step, 5,935). With ∇·v, an input
-// of the learned smoothing lengths, one lane sums the list in its order: the network takes it in 16 bits, and another
-// order of the sum moves some inputs by a whole step of those.
+// Four lanes to a particle: the two force passes of a step of 10,240 particles 21.5 µs (with a lane to a particle 49), of
+// 131,072 91 (116), of 262,144 165 (192), of 1,048,576 607 (623). With ∇·v, an input of the learned smoothing lengths,
+// one lane sums the list in its order: the network takes it in 16 bits, and another order of the sum moves some inputs
+// by a whole step of those.
 template <int KERNEL, bool GRAV, bool DIVV>
 __global__ void k_forces(int n, State st, const float4* __restrict__ fdata, const unsigned* __restrict__ nbr,
                          const unsigned* __restrict__ nbr_cnt, unsigned cap, unsigned sent,

@@ -254,9 +254,9 @@ __device__ __forceinline__ unsigned block_exclusive_scan(unsigned v, unsigned* s
 
 // Interleaved neighbour lists: warp-group g = t/32 owns a block of nbr_rows(cap) rows, a row holding four consecutive
 // entries of each of the 32 particles (16 bytes a particle, 512 a row): four lanes that read four consecutive entries of
-// each of eight particles read one 128-byte line. With rows of one entry (four lines for such a request) the forces took
-// 656 µs at 1,048,576 particles and 100 at 131,072, with these 607 and 91; the walk, which writes an entry at a time,
-// 4.96 and 4.98 ms.
+// each of eight particles read one 128-byte line. With rows of one entry (four lines for such a request) the two force
+// passes of a step took 656 µs at 1,048,576 particles and 100 at 131,072, with these 607 and 91; the walk, which writes an
+// entry at a time, 4.96 and 4.98 ms.
 __host__ __device__ __forceinline__ unsigned nbr_rows(unsigned cap) { return (cap + 3u) >> 2; }
 __host__ __device__ __forceinline__ size_t nbr_slot(unsigned t, unsigned k, unsigned cap) {
   return ((size_t)(t >> 5) * nbr_rows(cap) + (k >> 2)) * 128u + 4u * (t & 31u) + (k & 3u);

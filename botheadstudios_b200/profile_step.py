@@ -22,7 +22,7 @@ def main():
                     help="group walk: the local expansion's opening parameter (0 = off; default: the library's)")
     ap.add_argument("--precision", type=int, default=0, help="1 = node-relative hi/lo + compensated sums")
     ap.add_argument("--leaf", type=int, default=None, help="LBVH leaf size (default: the workload's)")
-    ap.add_argument("--walk-warps", type=int, default=0, help="warps per walk block (2, 4, 8; 0 = 4)")
+    ap.add_argument("--walk-warps", type=int, default=0, help="accepted (2, 4, 8) without effect: the walk chooses by size")
     ap.add_argument("--block", type=int, default=0, help="threads per block of the gather kernels (0 = 256)")
     ap.add_argument("--gravity", default=None, choices=["tree", "direct", "none"], help="override the gravity mode")
     ap.add_argument("--accuracy", type=int, default=0,
