@@ -63,6 +63,7 @@ struct SortSmem {
   unsigned gbin[SO_BINS];                  // where it goes
   unsigned long long warp[33];
   unsigned ticket;
+  unsigned finished;  // (not `ticket`: a warp may still be reading the ticket that ended its loop)
 };
 
 __device__ __forceinline__ unsigned long long scan_u64(unsigned long long v, unsigned long long* s_warp) {
@@ -290,9 +291,9 @@ __global__ void __launch_bounds__(SO_THREADS, 2) k_radix_sort(
     if (tid == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" :: "l"(&ctl->done[phase]) : "memory");
   }
   // the last block to run out of tickets leaves the control block ready for the next sort
-  if (tid == 0) S.ticket = atomicAdd(&ctl->finished, 1u);
+  if (tid == 0) S.finished = atomicAdd(&ctl->finished, 1u);
   __syncthreads();
-  if (S.ticket == gridDim.x - 1) {
+  if (S.finished == gridDim.x - 1) {
     for (int k = tid; k < SO_PASSES * SO_BINS; k += SO_THREADS) (&ctl->hist[0][0])[k] = 0u;
     if (tid <= SO_PASSES) ctl->done[tid] = 0u;
     if (tid == 0) {

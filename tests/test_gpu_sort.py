@@ -56,3 +56,13 @@ def test_sort_of_a_batch_keeps_the_impacts_apart(sizes):
     with GpuSph(len(p), gravity="none", leaf_size=16, max_neighbours=4) as s:
         s.upload_batch(p, offsets, M.eos_table(), 0.0)
         _check(s, p, offsets)
+
+
+@pytest.mark.parametrize("n", [5_000, 100_000])
+def test_sorts_in_a_row_stay_exact(n):
+    """Many blocks leave the ticket loop at different times, many times."""
+    p = _parts(n, 9)
+    with GpuSph(n, gravity="none", leaf_size=16, max_neighbours=4) as s:
+        s.upload(p, M.eos_table(), 0.0)
+        for _ in range(60):
+            _check(s, p, [0, n])
