@@ -37,18 +37,24 @@ struct SortCtl {
 constexpr int kSmallTiles = 64 * 2 * SO_THREADS;
 constexpr int kOneLaunchMax = 148 * 4 * SO_THREADS;
 
-// ---- the chain's workspace: [256][tiles] digit counts, 256 digit totals ----
+// ---- the chain's workspace: [256][tiles] digit counts, 256 digit totals, behind the tile words of the one launch. The
+// two forms share nothing: the one launch takes any word with its tag for a published count, and tags, like counts, are
+// small numbers.
 constexpr int RS_THREADS = 256;
 constexpr int RS_ITEMS = 8;
 constexpr int RS_TILE = RS_THREADS * RS_ITEMS;  // 2048 keys per tile
 constexpr int RS_WARPS = RS_THREADS / 32;
 
+constexpr int kMaxTiles = kOneLaunchMax / (4 * SO_THREADS);
+static_assert(kMaxTiles >= kSmallTiles / (2 * SO_THREADS), "no sort of one launch has more tiles");
+constexpr size_t kChainAt = kSortCtlBytes + kMaxTiles * kSortTileBytes;
+
 size_t sort_work_bytes(int n) {
-  const size_t m = n < 1 ? 1 : n, small = m < kSmallTiles ? m : kSmallTiles, one = m < kOneLaunchMax ? m : kOneLaunchMax;
-  const size_t t2 = (small + 2 * SO_THREADS - 1) / (2 * SO_THREADS), t4 = (one + 4 * SO_THREADS - 1) / (4 * SO_THREADS);
-  const size_t launch = kSortCtlBytes + (t2 > t4 ? t2 : t4) * kSortTileBytes;
-  const size_t chain = m > kOneLaunchMax ? kSortCtlBytes + 256 * sizeof(unsigned) * ((m + RS_TILE - 1) / RS_TILE + 1) : 0;
-  return launch > chain ? launch : chain;
+  const size_t m = n < 1 ? 1 : n;
+  if (m > kOneLaunchMax) return kChainAt + 256 * sizeof(unsigned) * ((m + RS_TILE - 1) / RS_TILE + 1);
+  const size_t small = m < kSmallTiles ? m : kSmallTiles;
+  const size_t t2 = (small + 2 * SO_THREADS - 1) / (2 * SO_THREADS), t4 = (m + 4 * SO_THREADS - 1) / (4 * SO_THREADS);
+  return kSortCtlBytes + (t2 > t4 ? t2 : t4) * kSortTileBytes;
 }
 static_assert(sizeof(SortCtl) <= kSortCtlBytes, "the control block fits its share of the workspace");
 static_assert(SO_BINS * 8 == kSortTileBytes, "a tile publishes one word for each digit");
@@ -466,7 +472,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(const unsigned long
 static int chain_sort(unsigned long long* const keys[2], unsigned* const vals[2], int n, int bits, void* work, int& src,
                       cudaStream_t s) {
   const int T = (n + RS_TILE - 1) / RS_TILE;
-  unsigned* hist = reinterpret_cast<unsigned*>(static_cast<unsigned char*>(work) + kSortCtlBytes);
+  unsigned* hist = reinterpret_cast<unsigned*>(static_cast<unsigned char*>(work) + kChainAt);
   unsigned* tot = hist + 256 * (size_t)T;
   src = 0;
   int launches = 0;

@@ -66,3 +66,12 @@ def test_sorts_in_a_row_stay_exact(n):
         s.upload(p, M.eos_table(), 0.0)
         for _ in range(60):
             _check(s, p, [0, n])
+
+
+def test_one_workspace_sorts_by_both_forms_in_turn():
+    """A context is refilled with fewer particles: the chain's counts must not pass for the one launch's tile words."""
+    with GpuSph(400_000, gravity="none", leaf_size=16, max_neighbours=4) as s:
+        for n in (400_000, 50_000, 200_000, 400_000, 300_000, 60_000, 304_000, 1_500, 303_104):
+            p = _parts(n, n + 3)
+            s.upload(p, M.eos_table(), 0.0)
+            _check(s, p, [0, n])
