@@ -71,6 +71,7 @@ EXPORTS = ["sph_config_default", "sph_create", "sph_destroy", "sph_upload", "sph
            "sph_set_av",
            "sph_set_omega", "sph_step_kdk", "sph_step_relax", "sph_eval_forces", "sph_readback_begin",
            "sph_readback_take", "sph_readback_into", "sph_sync", "sph_count", "sph_particle_buffer", "sph_diag", "sph_stream",
+           "sph_set_sort_polls",
            "sph_last_error", "sph_status_string", "sph_inspect", "sph_profile_enable", "sph_profile_read",
            "sph_gravity", "sph_gravity_direct64", "sph_gravity_tree_noalloc", "sph_dem_create", "sph_dem_destroy",
            "sph_dem_replace", "sph_dem_set_params", "sph_dem_step", "sph_dem_readback", "sph_dem_contacts",
@@ -157,6 +158,7 @@ def load():
     L.sph_diag.argtypes = [vp, C.POINTER(SphDiag)]
     L.sph_stream.argtypes = [vp]
     L.sph_stream.restype = vp
+    L.sph_set_sort_polls.argtypes = [vp, C.c_uint32]
     L.sph_last_error.argtypes = [vp]
     L.sph_last_error.restype = C.c_char_p
     L.sph_status_string.argtypes = [C.c_int]

@@ -558,12 +558,15 @@ __global__ void __launch_bounds__(kDmThreads) k_dm_compact(State st, const float
   }
 }
 
+// A sort's waits ran out: its result is no permutation, nothing that follows may use it, and the call returns the error.
+__device__ __forceinline__ bool unsorted(const unsigned* cnt) { return (cnt[C_ERR] & kFlagSortTimeout) != 0u; }
+
 __global__ void k_dm_gather(unsigned n, const unsigned* __restrict__ order, const float4* __restrict__ p0,
                             const float4* __restrict__ v0, const float2* __restrict__ r0, float4* __restrict__ p1,
                             float4* __restrict__ v1, float2* __restrict__ r1, unsigned* __restrict__ parent,
-                            unsigned* __restrict__ gcnt) {
+                            unsigned* __restrict__ gcnt, const unsigned* __restrict__ cnt) {
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  if (i >= n || unsorted(cnt)) return;
   const unsigned j = order[i];
   p1[i] = p0[j];
   v1[i] = v0[j];
@@ -633,6 +636,7 @@ __global__ void __launch_bounds__(kDmThreads) k_dm_link(unsigned n, int variant,
                                                         const float4* __restrict__ dpos,
                                                         const double* __restrict__ scal,
                                                         unsigned* __restrict__ parent, unsigned* __restrict__ cnt) {
+  if (unsorted(cnt)) return;
   const unsigned lane = threadIdx.x & 31u;
   const unsigned nwarps = (gridDim.x * blockDim.x) >> 5;
   const unsigned top = (1u << bits) - 1u;
@@ -688,9 +692,10 @@ __global__ void __launch_bounds__(kDmThreads) k_dm_link(unsigned n, int variant,
 }
 
 __global__ void k_dm_roots(unsigned n, unsigned* __restrict__ parent, unsigned* __restrict__ gcnt,
-                           unsigned long long* __restrict__ keys, unsigned* __restrict__ vals) {
+                           unsigned long long* __restrict__ keys, unsigned* __restrict__ vals,
+                           const unsigned* __restrict__ cnt) {
   const unsigned a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= n) return;
+  if (a >= n || unsorted(cnt)) return;
   const unsigned r = uf_find(parent, a);
   atomicAdd(&gcnt[r], 1u);
   keys[a] = r;
@@ -702,7 +707,7 @@ __global__ void k_dm_clumps(unsigned n, const unsigned long long* __restrict__ s
                             const unsigned* __restrict__ order, const unsigned* __restrict__ gcnt,
                             uint4* __restrict__ clump, unsigned* __restrict__ cnt) {
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  if (i >= n || unsorted(cnt)) return;
   const unsigned r = (unsigned)skeys[i];
   if (i > 0 && (unsigned)skeys[i - 1] == r) return;
   const unsigned s = gcnt[r];
@@ -1272,18 +1277,18 @@ int disk_measure(const Dev& d, unsigned off, unsigned m, const DiskCfg& c, DiskW
     k_dm_compact<<<nb, kDmThreads, 0, s>>>(st, d.rho, off, m, chunk, bits, w->cat, w->bcnt, w->scal, w->dpos[0],
                                            w->dvel[0], w->drp[0], w->keys[0], w->vals[0]);
     L += 1;
-    L += launch_radix_sort(w->keys, w->vals, (int)nd, 3 * bits, w->sort_work, w->cnt + C_ERR, src, s);
+    L += launch_radix_sort(w->keys, w->vals, (int)nd, 3 * bits, w->sort_work, d.sort_polls, w->cnt + C_ERR, src, s);
     const unsigned gb = (nd + 255) / 256;
     k_dm_gather<<<gb, 256, 0, s>>>(nd, w->vals[src], w->dpos[0], w->dvel[0], w->drp[0], w->dpos[1], w->dvel[1],
-                                   w->drp[1], w->parent, w->gcnt);
+                                   w->drp[1], w->parent, w->gcnt, w->cnt);
     const unsigned lb = (nd + 7) / 8;  // one warp per particle, grid-strided over at most 16 blocks per SM
     k_dm_link<<<lb < 2368u ? lb : 2368u, kDmThreads, 0, s>>>(nd, c.variant, bits, w->keys[src], w->dpos[1], w->scal,
                                                              w->parent, w->cnt);
-    k_dm_roots<<<gb, 256, 0, s>>>(nd, w->parent, w->gcnt, w->keys[0], w->vals[0]);
+    k_dm_roots<<<gb, 256, 0, s>>>(nd, w->parent, w->gcnt, w->keys[0], w->vals[0], w->cnt);
     L += 3;
-    L += launch_radix_sort(w->keys, w->vals, (int)nd, bits_of(nd), w->sort_work, w->cnt + C_ERR, src, s);
+    L += launch_radix_sort(w->keys, w->vals, (int)nd, bits_of(nd), w->sort_work, d.sort_polls, w->cnt + C_ERR, src, s);
     k_dm_gather<<<gb, 256, 0, s>>>(nd, w->vals[src], w->dpos[1], w->dvel[1], w->drp[1], w->dpos[0], w->dvel[0],
-                                   w->drp[0], nullptr, nullptr);
+                                   w->drp[0], nullptr, nullptr, w->cnt);
     k_dm_clumps<<<gb, 256, 0, s>>>(nd, w->keys[src], w->vals[src], w->gcnt, w->clump, w->cnt);
     const unsigned cb = nd / 2 < 1184u ? nd / 2 : 1184u;  // clumps <= nd / 2; blocks stride over them
     const unsigned sb = nd / 2 < 296u ? nd / 2 : 296u;  // two blocks of 1,024 threads per SM

@@ -9,8 +9,9 @@
 // memory. A phase waits until the previous one is complete. Tickets are drawn in order, so whatever a tile waits for is
 // held by a block that already runs: the launch needs no co-residency and any number of blocks. Ten-bit digits make
 // three passes of a 30-bit code; a digit's counters are 16-bit in shared memory.
-// Every wait is bounded: after kSortPolls polls the block raises kFlagSortTimeout and goes on (the scatter checks its
-// bounds), so a fault in the protocol shows as a flag and not as a hang.
+// Every wait is bounded: after Dev::sort_polls polls the block raises kFlagSortTimeout and goes on (the scatter checks its
+// bounds), so a fault in the protocol shows as a flag and not as a hang. What comes out is then no permutation, and the
+// control block says so (SortEnd): the callers do without it.
 #include "sph_kernels.cuh"
 
 namespace sphb {
@@ -20,12 +21,12 @@ constexpr int SO_WARPS = SO_THREADS / 32;
 constexpr int SO_BITS = 10;
 constexpr int SO_BINS = 1 << SO_BITS;
 constexpr int SO_PASSES = 7;  // 64-bit keys
-constexpr unsigned kSortPolls = 1u << 21;
 constexpr int SO_LOOK = 8;    // predecessors read at a time
 
 // The sort's control block: zero before the first sort, left ready for the next one by the last block to finish.
 struct SortCtl {
-  unsigned ticket, finished, epoch, pad;
+  unsigned ticket, finished;
+  SortEnd end;
   unsigned done[SO_PASSES + 1];      // tiles complete in each phase
   unsigned hist[SO_PASSES][SO_BINS];
 };
@@ -111,8 +112,8 @@ __device__ __forceinline__ unsigned same_digit(unsigned d, bool in) {
 }
 
 // Polls *p (written by other blocks) until it reaches `want`.
-__device__ __forceinline__ bool wait_count(const unsigned* p, unsigned want) {
-  for (unsigned k = 0; k < kSortPolls; ++k) {
+__device__ __forceinline__ bool wait_count(const unsigned* p, unsigned want, unsigned limit) {
+  for (unsigned k = 0; k < limit; ++k) {
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     if (v >= want) return true;
@@ -122,7 +123,8 @@ __device__ __forceinline__ bool wait_count(const unsigned* p, unsigned want) {
 
 // Counts of digits 2t and 2t + 1 in the tiles before `tile`. The published words are tag << 32 | state << 30 | count,
 // state 1 the tile's own count, 2 the count up to and including the tile; SO_LOOK tiles' words are read at a time.
-__device__ __forceinline__ uint2 look_back(const unsigned long long* status, int tile, int t, unsigned tag, bool& ok) {
+__device__ __forceinline__ uint2 look_back(const unsigned long long* status, int tile, int t, unsigned tag, unsigned limit,
+                                           bool& ok) {
   uint2 before = make_uint2(0u, 0u);
   int ja = tile - 1, jb = tile - 1;
   for (unsigned polls = 0; ja >= 0 || jb >= 0;) {
@@ -144,7 +146,7 @@ __device__ __forceinline__ uint2 look_back(const unsigned long long* status, int
         jb = ((unsigned)b[k] >> 30) == 2u ? -1 : jb - 1;
       }
     }
-    if (ja == a0 && jb == b0 && ++polls > kSortPolls) {
+    if (ja == a0 && jb == b0 && ++polls > limit) {
       ok = false;
       break;
     }
@@ -155,14 +157,18 @@ __device__ __forceinline__ uint2 look_back(const unsigned long long* status, int
 template <bool MORTON, int SO_ITEMS>
 __global__ void __launch_bounds__(SO_THREADS, 2) k_radix_sort(
     int n, int T, int passes, unsigned long long* keys0, unsigned long long* keys1, unsigned* vals0, unsigned* vals1,
-    SortCtl* ctl, unsigned long long* status, unsigned* flags, const float4* __restrict__ pos,
+    SortCtl* ctl, unsigned long long* status, unsigned polls, unsigned* flags, const float4* __restrict__ pos,
     const unsigned* __restrict__ id, const unsigned* __restrict__ seg, const Seg* __restrict__ segs) {
   extern __shared__ __align__(16) unsigned char so_raw[];
   SortSmem<SO_ITEMS>& S = *reinterpret_cast<SortSmem<SO_ITEMS>*>(so_raw);
   constexpr int SO_TILE = SO_THREADS * SO_ITEMS;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const unsigned lt_mask = (1u << lane) - 1u;
-  const unsigned epoch = ctl->epoch;
+  const unsigned epoch = ctl->end.epoch;
+  const auto timed_out = [&] {
+    atomicOr(flags, kFlagSortTimeout);
+    atomicExch(&ctl->end.failed, epoch + 1u);
+  };
   const unsigned total = (unsigned)(T * (passes + 1));
   unsigned next = 0;  // thread 0: the ticket after this one, drawn while this one is worked on
   if (tid == 0) next = atomicAdd(&ctl->ticket, 1u);
@@ -212,7 +218,7 @@ __global__ void __launch_bounds__(SO_THREADS, 2) k_radix_sort(
       unsigned long long* kout = q & 1 ? keys0 : keys1;
       unsigned* vout = q & 1 ? vals0 : vals1;
       for (int k = tid; k < SO_WARPS * SO_BINS / 2; k += SO_THREADS) reinterpret_cast<unsigned*>(&S.wcnt[0][0])[k] = 0u;
-      if (tid == 0 && !wait_count(&ctl->done[phase - 1], (unsigned)T)) atomicOr(flags, kFlagSortTimeout);
+      if (tid == 0 && !wait_count(&ctl->done[phase - 1], (unsigned)T, polls)) timed_out();
       __syncthreads();
       unsigned long long key[SO_ITEMS];
       unsigned val[SO_ITEMS], rank[SO_ITEMS];
@@ -259,8 +265,8 @@ __global__ void __launch_bounds__(SO_THREADS, 2) k_radix_sort(
       const unsigned h0 = (unsigned)hist2, h1 = (unsigned)(hist2 >> 32);
       const unsigned long long ex = scan_u64(((unsigned long long)(h0 + h1) << 32) | (c0 + c1), S.warp);
       bool ok = true;
-      const uint2 before = look_back(status, tile, tid, tag, ok);
-      if (!ok) atomicOr(flags, kFlagSortTimeout);
+      const uint2 before = look_back(status, tile, tid, tag, polls, ok);
+      if (!ok) timed_out();
       if (tile > 0) {
         mine[0] = word | (2u << 30) | (before.x + c0);
         mine[1] = word | (2u << 30) | (before.y + c1);
@@ -305,14 +311,14 @@ __global__ void __launch_bounds__(SO_THREADS, 2) k_radix_sort(
     if (tid == 0) {
       ctl->ticket = 0u;
       ctl->finished = 0u;
-      ctl->epoch = epoch + 1u;
+      ctl->end.epoch = epoch + 1u;
     }
   }
 }
 
 template <bool MORTON, int ITEMS>
 static int radix_sort(int n, int bits, unsigned long long* const keys[2], unsigned* const vals[2], void* work,
-                      unsigned* flags, const State* st, const Seg* segs, cudaStream_t s) {
+                      unsigned polls, unsigned* flags, const State* st, const Seg* segs, cudaStream_t s) {
   static std::atomic<unsigned long long> attr{0};
   smem_limit_per_device(k_radix_sort<MORTON, ITEMS>, (int)sizeof(SortSmem<ITEMS>), attr);
   const int tile = SO_THREADS * ITEMS, T = (n + tile - 1) / tile, passes = (bits + SO_BITS - 1) / SO_BITS;
@@ -320,16 +326,16 @@ static int radix_sort(int n, int bits, unsigned long long* const keys[2], unsign
   SortCtl* ctl = static_cast<SortCtl*>(work);
   unsigned long long* status = reinterpret_cast<unsigned long long*>(static_cast<unsigned char*>(work) + kSortCtlBytes);
   k_radix_sort<MORTON, ITEMS><<<grid, SO_THREADS, sizeof(SortSmem<ITEMS>), s>>>(
-      n, T, passes, keys[0], keys[1], vals[0], vals[1], ctl, status, flags, st ? st->pos_h : nullptr,
+      n, T, passes, keys[0], keys[1], vals[0], vals[1], ctl, status, polls, flags, st ? st->pos_h : nullptr,
       st ? st->id : nullptr, st ? st->seg : nullptr, segs);
   return passes & 1;
 }
 
 template <bool MORTON>
 static int one_launch(int n, int bits, unsigned long long* const keys[2], unsigned* const vals[2], void* work,
-                      unsigned* flags, const State* st, const Seg* segs, cudaStream_t s) {
-  if (n <= kSmallTiles) return radix_sort<MORTON, 2>(n, bits, keys, vals, work, flags, st, segs, s);
-  return radix_sort<MORTON, 4>(n, bits, keys, vals, work, flags, st, segs, s);
+                      unsigned polls, unsigned* flags, const State* st, const Seg* segs, cudaStream_t s) {
+  if (n <= kSmallTiles) return radix_sort<MORTON, 2>(n, bits, keys, vals, work, polls, flags, st, segs, s);
+  return radix_sort<MORTON, 4>(n, bits, keys, vals, work, polls, flags, st, segs, s);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -487,21 +493,23 @@ static int chain_sort(unsigned long long* const keys[2], unsigned* const vals[2]
 }
 
 int launch_radix_sort(unsigned long long* const keys[2], unsigned* const vals[2], int n, int bits, void* work,
-                      unsigned* flags, int& src, cudaStream_t s) {
+                      unsigned polls, unsigned* flags, int& src, cudaStream_t s) {
   src = 0;
   if (n <= 1) return 0;
   if (n > kOneLaunchMax) return chain_sort(keys, vals, n, bits, work, src, s);
-  src = one_launch<false>(n, bits, keys, vals, work, flags, nullptr, nullptr, s);
+  src = one_launch<false>(n, bits, keys, vals, work, polls, flags, nullptr, nullptr, s);
   return 1;
 }
 
-int launch_morton_sort(const Dev& d, int& src, cudaStream_t s) {
+int launch_morton_sort(const Dev& d, int& src, const SortEnd*& end, cudaStream_t s) {
+  end = nullptr;  // the chain waits for nothing
   const State& in = d.st[d.cur];
   if (d.n > kOneLaunchMax) {
     k_keys<<<(d.n + 255) / 256, 256, 0, s>>>(in.pos_h, in.id, in.seg, d.n, d.segs, d.keys[0], d.vals[0]);
     return 1 + chain_sort(d.keys, d.vals, d.n, 30 + d.segbits, d.sort_work, src, s);
   }
-  src = one_launch<true>(d.n, 30 + d.segbits, d.keys, d.vals, d.sort_work, &d.P->flags, &in, d.segs, s);
+  end = &static_cast<SortCtl*>(d.sort_work)->end;
+  src = one_launch<true>(d.n, 30 + d.segbits, d.keys, d.vals, d.sort_work, d.sort_polls, &d.P->flags, &in, d.segs, s);
   return 1;
 }
 

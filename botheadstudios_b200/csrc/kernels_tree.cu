@@ -90,15 +90,19 @@ static int launch_bbox(const Dev& d, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------------------------------------
-// Permutation of the particle state into the new order; leaf cluster codes (gpu_gravity.rs:366).
+// Permutation of the particle state into the new order; leaf cluster codes (gpu_gravity.rs:366). After a sort whose waits
+// ran out the particles stay where they are and the leaves are coded in that order: any order gives a valid tree, with
+// larger boxes, so what follows stays in bounds and its results stay good.
 // ---------------------------------------------------------------------------------------------------
 __global__ void k_permute(int n, int L, const unsigned* __restrict__ order,
                           const unsigned long long* __restrict__ skeys, const unsigned* __restrict__ leaf_start,
                           State in, State out, float4* __restrict__ body,
-                          unsigned long long* __restrict__ leaf_codes) {
+                          unsigned long long* __restrict__ leaf_codes, const SortEnd* __restrict__ end,
+                          const Seg* __restrict__ segs) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
-  const unsigned o = order[t];
+  const bool sorted = !end || end->epoch != end->failed;
+  const unsigned o = sorted ? order[t] : (unsigned)t;
   const float4 p = in.pos_h[o];
   const float m = in.mass[o];
   out.pos_h[t] = p;
@@ -112,7 +116,15 @@ __global__ void k_permute(int n, int L, const unsigned* __restrict__ order,
   out.id[t] = in.id[o];
   out.seg[t] = in.seg[o];
   body[t] = make_float4(p.x, p.y, p.z, m);
-  if (t < L) leaf_codes[t] = skeys[leaf_start[t]];
+  if (t < L) {
+    const unsigned first = leaf_start[t];
+    if (sorted) {
+      leaf_codes[t] = skeys[first];
+    } else {
+      const unsigned sg = in.seg[first];
+      leaf_codes[t] = (unsigned long long)sg << 30 | ((unsigned)t - segs[sg].loff);
+    }
+  }
 }
 
 // The sort order is (segment, code, original index): the sort is stable and starts out in original-index order
@@ -123,10 +135,11 @@ int launch_sort_permute(Dev& d, bool need_bbox, cudaStream_t s) {
   const State& in = d.st[d.cur];
   const State& out = d.st[d.cur ^ 1];
   int src = 0;
-  const int sorts = launch_morton_sort(d, src, s);
+  const SortEnd* end;
+  const int sorts = launch_morton_sort(d, src, end, s);
   // vals[src] = old slot of each sorted position; keys[src] = sorted keys
   k_permute<<<(n + 255) / 256, 256, 0, s>>>(n, d.L, d.vals[src], d.keys[src], d.leaf_start, in, out, d.body,
-                                            d.leaf_codes);
+                                            d.leaf_codes, end, d.segs);
   d.cur ^= 1;
   d.sorted = src;
   return box + sorts + 1;

@@ -795,6 +795,15 @@ sph_status sph_particle_buffer(sph_ctx* ctx, void** device_ptr) {
 }
 
 void* sph_stream(sph_ctx* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
+sph_status sph_set_sort_polls(sph_ctx* ctx, uint32_t polls) {
+  if (!ctx) return SPH_ERR_INVALID;
+  cudaSetDevice(ctx->device);
+  CK(cudaStreamSynchronize(ctx->stream));
+  drop_graphs(ctx);
+  ctx->d.sort_polls = ctx->g.sort_polls = polls;
+  return SPH_OK;
+}
+
 const char* sph_last_error(const sph_ctx* ctx) { return ctx ? ctx->err.c_str() : "null context"; }
 
 sph_status sph_body_bulk(sph_ctx* ctx, uint32_t prov, double centre[3], double* mass, double* radius) {

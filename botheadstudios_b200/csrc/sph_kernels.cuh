@@ -56,6 +56,12 @@ struct Seg {
 static_assert(sizeof(Seg) == 72, "Seg is one 72-byte record");
 constexpr unsigned kNoSeg = 0xffffffffu;
 
+constexpr unsigned kSortPolls = 1u << 21;  // about a second
+// How a workspace's last one-launch sort ended: its waits ran out if the two are equal.
+struct SortEnd {
+  unsigned epoch, failed;
+};
+
 // The table of a single impact: an empty bounding box, no simulated time.
 __device__ __forceinline__ void write_single_segment(Seg* segs, int n, int L, float soft2, double dt) {
   Seg a;
@@ -165,6 +171,7 @@ struct Dev {
   unsigned long long* keys[2] = {nullptr, nullptr};
   unsigned* vals[2] = {nullptr, nullptr};
   void* sort_work = nullptr;    // the sort's control block and published tile counts (sort_work_bytes)
+  unsigned sort_polls = kSortPolls;  // polls of one of the sort's waits
   int sorted = 0;               // the keys/vals buffer that holds the last sort's result
   int nseg = 1;
   int segbits = 0;                 // sort-key bits of the segment index (0 for one segment)
@@ -261,13 +268,14 @@ int launch_tree(const Dev& d, const Cfg& c, float theta, cudaStream_t s);  // li
 int half_leaf(const Dev& d, const Cfg& c);
 // Stable LSD radix sort (kernels_sort.cu) on the low `bits` key bits; the result lands in buffer `src`. `work`:
 // sort_work_bytes(n) of device memory, zero before its first sort and used by one sort at a time; a sort whose
-// waits run out raises kFlagSortTimeout in *flags.
+// waits run out after `polls` polls raises kFlagSortTimeout in *flags; its result is then no permutation.
 constexpr size_t kSortCtlBytes = 32768, kSortTileBytes = 8192, kSortTileMin = 1024;
 size_t sort_work_bytes(int n);
 int launch_radix_sort(unsigned long long* const keys[2], unsigned* const vals[2], int n, int bits, void* work,
-                      unsigned* flags, int& src, cudaStream_t s);
-// Morton keys of the current state (segment << 30 | code), sorted with the particles' slots
-int launch_morton_sort(const Dev& d, int& src, cudaStream_t s);
+                      unsigned polls, unsigned* flags, int& src, cudaStream_t s);
+// Morton keys of the current state (segment << 30 | code), sorted with the particles' slots; `end`: device memory that
+// says whether the sort's waits ran out, or null for a sort without any
+int launch_morton_sort(const Dev& d, int& src, const SortEnd*& end, cudaStream_t s);
 
 // ---- gravity ---------------------------------------------------------------------------------------
 int launch_gravity_tree(const Dev& d, const Cfg& c, cudaStream_t s);

@@ -265,6 +265,11 @@ sph_status sph_measure_default(sph_measure_cfg* cfg);
 sph_status sph_measure_disk(sph_ctx* ctx, uint32_t impact, const sph_measure_cfg* cfg, sph_disk_measure* out);
 /* The context's CUDA stream (cudaStream_t), for callers that order their own work after the step. */
 void* sph_stream(sph_ctx* ctx);
+/* Polls after which a wait inside the Morton sort gives up (2^21 at creation, about a second; 0: at once, for testing that
+ * path). A rebuild whose sort gave up keeps the particles in the order they had: its results stay valid, its walk is
+ * slower, and from then on sph_diag returns SPH_ERR_TIMEOUT (with its output filled). sph_measure_disk fails with
+ * SPH_ERR_TIMEOUT when one of its own sorts gives up. */
+sph_status sph_set_sort_polls(sph_ctx* ctx, uint32_t polls);
 const char* sph_last_error(const sph_ctx* ctx);
 const char* sph_status_string(sph_status s);
 
