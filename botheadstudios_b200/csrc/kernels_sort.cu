@@ -18,18 +18,7 @@ namespace sphb {
 
 constexpr int SO_THREADS = 512;
 constexpr int SO_WARPS = SO_THREADS / 32;
-constexpr int SO_BITS = 10;
-constexpr int SO_BINS = 1 << SO_BITS;
-constexpr int SO_PASSES = 7;  // 64-bit keys
 constexpr int SO_LOOK = 8;    // predecessors read at a time
-
-// The sort's control block: zero before the first sort, left ready for the next one by the last block to finish.
-struct SortCtl {
-  unsigned ticket, finished;
-  SortEnd end;
-  unsigned done[SO_PASSES + 1];      // tiles complete in each phase
-  unsigned hist[SO_PASSES][SO_BINS];
-};
 
 // Keys to a thread. A tile is worked on by one SM, whose shared memory and stores bound it (8,192 keys take 12 µs a
 // pass), so small sorts take small tiles on many SMs; a tile's look-back reads the counts of every tile before it, so
@@ -57,7 +46,6 @@ size_t sort_work_bytes(int n) {
   const size_t t2 = (small + 2 * SO_THREADS - 1) / (2 * SO_THREADS), t4 = (m + 4 * SO_THREADS - 1) / (4 * SO_THREADS);
   return kSortCtlBytes + (t2 > t4 ? t2 : t4) * kSortTileBytes;
 }
-static_assert(sizeof(SortCtl) <= kSortCtlBytes, "the control block fits its share of the workspace");
 static_assert(SO_BINS * 8 == kSortTileBytes, "a tile publishes one word for each digit");
 
 template <int ITEMS>

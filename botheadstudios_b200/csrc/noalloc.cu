@@ -186,8 +186,18 @@ Dev carve_dev(unsigned char* base, uint32_t K) {
   return d;
 }
 
-// Everything the walk reads from DevParams, written on the device (no host copy), counters cleared; the segment table.
-__global__ void k_noalloc_params(DevParams* P, Seg* segs, int n, int L, float soft2, float G, float theta) {
+// Everything the walk reads from DevParams, written on the device (no host copy), counters cleared; the segment table. And
+// what the sort and the tree keep in the scratch between calls, as they leave it at their end: calls that overlapped in
+// spite of the interface spoil each other's results, but not those of the calls after them. (The sort's epoch goes on: words
+// that an overlapped sort published carry an older one.)
+__global__ void __launch_bounds__(1024) k_noalloc_params(DevParams* P, Seg* segs, int n, int L, float soft2, float G,
+                                                         float theta, SortCtl* sort, unsigned long long* slots) {
+  for (int k = threadIdx.x; k < SO_PASSES * SO_BINS; k += blockDim.x) (&sort->hist[0][0])[k] = 0u;
+  for (int k = threadIdx.x; k < L; k += blockDim.x) slots[k] = 0ull;
+  if (threadIdx.x <= SO_PASSES) sort->done[threadIdx.x] = 0u;
+  if (threadIdx.x != 0) return;
+  sort->ticket = sort->finished = 0u;
+  ++sort->end.epoch;
   DevParams p;
   memset(&p, 0, sizeof(p));
   p.G = G;
@@ -262,7 +272,8 @@ extern "C" sph_status sph_gravity_tree_noalloc(const void* d_bodies4, uint32_t n
   c.quad = (int)multipole;
   c.mac = SPH_MAC_GROUP;
   c.local_theta = kLocalThetaDefault;  // the walk sph_gravity runs with the default configuration
-  k_noalloc_params<<<1, 1, 0, s>>>(d.P, d.segs, d.n, d.L, softening * softening, (float)G, theta);
+  k_noalloc_params<<<1, 1024, 0, s>>>(d.P, d.segs, d.n, d.L, softening * softening, (float)G, theta,
+                                      static_cast<SortCtl*>(d.sort_work), d.slots);
   k_noalloc_load<<<(n + 255) / 256, 256, 0, s>>>(static_cast<const float4*>(d_bodies4), (int)n, d.st[0], d.segs);
   launch_segments(d, s);
   launch_sort_permute(d, false, s);

@@ -61,6 +61,14 @@ constexpr unsigned kSortPolls = 1u << 21;  // about a second
 struct SortEnd {
   unsigned epoch, failed;
 };
+constexpr int SO_BITS = 10, SO_BINS = 1 << SO_BITS, SO_PASSES = 7;  // digits; passes of a 64-bit key
+// The one-launch sort's control block: zero before the first sort, left ready for the next one by the last block to finish.
+struct SortCtl {
+  unsigned ticket, finished;
+  SortEnd end;
+  unsigned done[SO_PASSES + 1];      // tiles complete in each phase
+  unsigned hist[SO_PASSES][SO_BINS];
+};
 
 // The table of a single impact: an empty bounding box, no simulated time.
 __device__ __forceinline__ void write_single_segment(Seg* segs, int n, int L, float soft2, double dt) {
@@ -270,6 +278,7 @@ int half_leaf(const Dev& d, const Cfg& c);
 // sort_work_bytes(n) of device memory, zero before its first sort and used by one sort at a time; a sort whose
 // waits run out after `polls` polls raises kFlagSortTimeout in *flags; its result is then no permutation.
 constexpr size_t kSortCtlBytes = 32768, kSortTileBytes = 8192, kSortTileMin = 1024;
+static_assert(sizeof(SortCtl) <= kSortCtlBytes, "the control block fits its share of the workspace");
 size_t sort_work_bytes(int n);
 int launch_radix_sort(unsigned long long* const keys[2], unsigned* const vals[2], int n, int bits, void* work,
                       unsigned polls, unsigned* flags, int& src, cudaStream_t s);

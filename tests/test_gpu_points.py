@@ -115,3 +115,26 @@ def test_point_walk_matches_its_definition(n, leaf, quad):
         assert np.isfinite(got).all()
         err = math.sqrt(((got - want) ** 2).sum() / max((want**2).sum(), 1e-300))
         assert err < 1e-5, (theta, err)
+
+
+def test_allocation_free_calls_in_a_row_leave_the_scratch_as_they_found_it():
+    """Every call resets what the sort and the tree keep between calls, so any sequence of sizes repeats its results."""
+    import ctypes as C
+
+    import torch
+
+    from botheadstudios_b200 import _lib
+
+    L = _lib.load()
+    first = {}
+    for n in (65_536, 33, 20_000, 65_536, 1, 33, 1_025, 20_000, 1_025, 1, 65_536):
+        _, pos, mass = cloud(n, 77)
+        body = torch.tensor(np.concatenate([pos, mass[:, None]], 1).astype(np.float32), device="cuda:0")
+        out = torch.full((n, 4), float("nan"), dtype=torch.float32, device="cuda:0")
+        s = torch.cuda.current_stream(0)
+        assert L.sph_gravity_tree_noalloc(C.c_void_p(body.data_ptr()), n, G, SOFT, 0.5, 8, 1, C.c_void_p(out.data_ptr()),
+                                          C.c_void_p(s.cuda_stream)) == _lib.SPH_OK
+        s.synchronize()
+        a = out.cpu().numpy()
+        assert np.isfinite(a).all()
+        assert np.array_equal(a, first.setdefault(n, a))
