@@ -238,8 +238,8 @@ __global__ void __launch_bounds__(PT_WARPS * 32) k_point_walk(
 
 template <bool QUAD>
 static void point_walk(const Dev& d, const Cfg& c, cudaStream_t s) {
-  static std::atomic<unsigned long long> attr{0};
-  smem_limit_per_device(k_point_walk<QUAD>, (int)sizeof(PointSmem), attr);
+  static SmemLimit attr;
+  smem_limit(k_point_walk<QUAD>, (int)sizeof(PointSmem), attr);
   k_point_walk<QUAD><<<(d.n + 31) / 32, PT_WARPS * 32, sizeof(PointSmem), s>>>(
       d.body, d.n, d.L, d.leaf_start, d.segs, d.left, d.right, d.ncom, d.nbmin, d.nbmax, d.nq0, d.nq1, d.P, d.grav,
       c.walk_stack > 0 && c.walk_stack < PT_STACK ? c.walk_stack : PT_STACK, half_leaf(d, c), d.hcom, d.hq0, d.hq1,

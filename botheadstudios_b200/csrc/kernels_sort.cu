@@ -307,8 +307,8 @@ __global__ void __launch_bounds__(SO_THREADS, 2) k_radix_sort(
 template <bool MORTON, int ITEMS>
 static int radix_sort(int n, int bits, unsigned long long* const keys[2], unsigned* const vals[2], void* work,
                       unsigned polls, unsigned* flags, const State* st, const Seg* segs, cudaStream_t s) {
-  static std::atomic<unsigned long long> attr{0};
-  smem_limit_per_device(k_radix_sort<MORTON, ITEMS>, (int)sizeof(SortSmem<ITEMS>), attr);
+  static SmemLimit attr;
+  smem_limit(k_radix_sort<MORTON, ITEMS>, (int)sizeof(SortSmem<ITEMS>), attr);
   const int tile = SO_THREADS * ITEMS, T = (n + tile - 1) / tile, passes = (bits + SO_BITS - 1) / SO_BITS;
   const int grid = T < 2 * 148 ? T : 2 * 148;
   SortCtl* ctl = static_cast<SortCtl*>(work);

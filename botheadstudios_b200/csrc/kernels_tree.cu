@@ -571,8 +571,8 @@ static void tree_build(const Dev& d, const NodeArrays& nodes, float theta, int h
   const int most = TB_THREADS * d.K, staged = most + (most >> 4) + 1;
   const size_t part = (size_t)staged * (sizeof(float4) + sizeof(float));
   const size_t smem = part > sizeof(TreeSmem) ? part : sizeof(TreeSmem);
-  static std::atomic<unsigned long long> attr{0};
-  smem_limit_per_device(k_tree_build<QUAD>, (TB_THREADS * 34 + 1) * 20, attr);  // leaves of 32
+  static SmemLimit attr;
+  smem_limit(k_tree_build<QUAD>, (TB_THREADS * 34 + 1) * 20, attr);  // leaves of 32
   k_tree_build<QUAD><<<(d.L + TB_RUN - 1) / TB_RUN, TB_THREADS, smem, s>>>(
       d.body, d.s().pos_h, d.leaf_start, d.L, d.leaf_codes, d.segs, d.left, d.right, d.parent, d.slots, nodes, theta, half,
       d.hcom, d.hq0, d.hq1, d.hrc, staged);

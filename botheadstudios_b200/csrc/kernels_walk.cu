@@ -1147,8 +1147,8 @@ template <int F, bool GRAV, bool QUAD, bool NBR, bool HILO, int OUT>
 static int walk_class(const Dev& d, const Cfg& c, int first, int count, cudaStream_t s) {
   if (count <= 0) return 0;
   const size_t smem = sizeof(WalkSmem<F>);
-  static std::atomic<unsigned long long> attr{0};
-  smem_limit_per_device(k_tree_walk<F, GRAV, QUAD, NBR, HILO, OUT>, (int)smem, attr);
+  static SmemLimit attr;
+  smem_limit(k_tree_walk<F, GRAV, QUAD, NBR, HILO, OUT>, (int)smem, attr);
   const State& st = d.s();
   constexpr int most = WalkSmem<F>::STACK;
   k_tree_walk<F, GRAV, QUAD, NBR, HILO, OUT><<<count, F * 32, smem, s>>>(

@@ -645,8 +645,8 @@ int launch_mlp_pack(const float* params, MlpPacked* out, cudaStream_t s) {
 
 int launch_mlp_propose(const Dev& d, const MlpPacked* w, const MlpFeatureArgs& fa, const float* divv, float* rec,
                        float* dh, bool apply, cudaStream_t s) {
-  static std::atomic<unsigned long long> attr{0};
-  smem_limit_per_device(k_mlp_propose, TC_SMEM, attr);
+  static SmemLimit attr;
+  smem_limit(k_mlp_propose, TC_SMEM, attr);
   const int tiles = (d.n + ROWS - 1) / ROWS;
   const int cap = propose_grid();
   const int grid = tiles < cap ? tiles : cap;
@@ -656,8 +656,8 @@ int launch_mlp_propose(const Dev& d, const MlpPacked* w, const MlpFeatureArgs& f
 }
 
 int launch_mlp_forward(const MlpPacked* w, const float* x, int n, float* out, unsigned* err, cudaStream_t s) {
-  static std::atomic<unsigned long long> attr{0};
-  smem_limit_per_device(k_mlp_forward, TC_SMEM, attr);
+  static SmemLimit attr;
+  smem_limit(k_mlp_forward, TC_SMEM, attr);
   const int tiles = (n + ROWS - 1) / ROWS;
   const int cap = propose_grid();
   const int grid = tiles < cap ? tiles : cap;
@@ -690,8 +690,8 @@ size_t mlp_part_floats(int m) { return (size_t)mlp_train_ctas(m) * MLP_PART; }
 
 int launch_mlp_train_batch(const MlpPacked* w, const float* x, const float* t, const unsigned* idx, int m,
                            float denom, float* part, unsigned* err, cudaStream_t s) {
-  static std::atomic<unsigned long long> attr{0};
-  smem_limit_per_device(k_mlp_train_tc, (int)sizeof(TrainTcSmem), attr);
+  static SmemLimit attr;
+  smem_limit(k_mlp_train_tc, (int)sizeof(TrainTcSmem), attr);
   launch_overlapped(k_mlp_train_tc, mlp_train_ctas(m), TT_THREADS, sizeof(TrainTcSmem), s, w, x, t, idx, m, denom, part,
                     err);
   return 1;

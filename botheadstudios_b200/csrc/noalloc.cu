@@ -86,7 +86,8 @@ const CtxFns& ctx_fns() {
   return fns;
 }
 
-// Id of the calling thread's current context, 0 when there is none (or the driver cannot say).
+}  // namespace
+
 unsigned long long current_ctx_id() {
   const CtxFns& f = ctx_fns();
   if (!f.get_current || !f.get_id) return 0;
@@ -95,6 +96,9 @@ unsigned long long current_ctx_id() {
   unsigned long long id = 0;
   return f.get_id(c, &id) == CUDA_SUCCESS ? id : 0;
 }
+
+namespace {
+
 
 // Device address of the scratch array for the current device and context. The lookup runs with the device
 // current, on the first call in each context; during a stream capture no lookup is made (the capture must

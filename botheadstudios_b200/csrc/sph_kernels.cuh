@@ -8,17 +8,26 @@
 
 namespace sphb {
 
-// Raises a kernel's dynamic shared-memory limit on the calling thread's current device, once per device: the
-// attribute belongs to the device, so contexts on several GPUs in one process each need it. `done` holds one
-// bit per device ordinal (below 64); two threads racing here both set the same value, which is harmless.
+// Id of the calling thread's current device context, 0 when there is none (or the driver cannot say). Ids are not used
+// again, so what is remembered under one is not taken for another's after a cudaDeviceReset.
+unsigned long long current_ctx_id();
+
+// Raises a kernel's dynamic shared-memory limit in the calling thread's current device context, once for each: the limit
+// goes with the context, so contexts on several GPUs of a process each need it, and one that follows a reset needs it
+// again. `done` holds the id of the context of each device ordinal (below 64) that has it; two threads racing here both
+// set the same value, which is harmless.
+struct SmemLimit {
+  std::atomic<unsigned long long> ctx[64] = {};
+};
 template <typename Kernel>
-inline void smem_limit_per_device(Kernel kernel, int bytes, std::atomic<unsigned long long>& done) {
+inline void smem_limit(Kernel kernel, int bytes, SmemLimit& done) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return;
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (done.load(std::memory_order_acquire) & bit) return;
+  std::atomic<unsigned long long>& slot = done.ctx[dev & 63];
+  const unsigned long long id = current_ctx_id();
+  if (id != 0 && slot.load(std::memory_order_acquire) == id) return;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
-    done.fetch_or(bit, std::memory_order_release);
+    slot.store(current_ctx_id(), std::memory_order_release);  // (the call makes a context if there was none)
 }
 
 // Particle state, structure-of-arrays, kept in Morton (LBVH leaf) order between force evaluations.
