@@ -5,6 +5,7 @@
 // computes the weight gradients as tcgen05 GEMMs over a tile's 128 samples; Adam updates an FP32 master copy.
 #include <cstdint>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -717,32 +718,38 @@ using namespace sphb;
 
 namespace {
 
-// The calls below allocate from a pool of their own for each device, which keeps up to 64 MB of what they free for the
-// next call and gives the rest back (cudaMalloc and cudaFree of a call's buffers took 0.4-0.7 ms of a 2 ms epoch of
-// 100,000 samples, and milliseconds on a busy host). Stream order on the default stream makes it safe between threads.
+// The calls below allocate from a pool of their own for each device context, which keeps up to 64 MB of what they free for
+// the next call and gives the rest back (cudaMalloc and cudaFree of a call's buffers took 0.4-0.7 ms of a 2 ms epoch of
+// 100,000 samples, and milliseconds on a busy host). A pool ends with its context: after a cudaDeviceReset the next call
+// makes another. Stream order on the default stream makes it safe between threads.
 constexpr unsigned long long kPoolKeeps = 64ull << 20;
 
 cudaError_t call_pool(cudaMemPool_t* pool) {
   static std::mutex mu;
-  static cudaMemPool_t pools[64] = {};
+  static std::map<unsigned long long, cudaMemPool_t> pools;  // by the context's id
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess && current_ctx_id() == 0) e = cudaFree(nullptr);  // the device's context, if there is none yet
   if (e != cudaSuccess) return e;
-  if (dev >= 64) return cudaErrorInvalidDevice;
+  const unsigned long long id = current_ctx_id();
+  if (id == 0) return cudaDeviceGetDefaultMemPool(pool, dev);  // nothing to remember a pool under
   std::lock_guard<std::mutex> lock(mu);
-  if (!pools[dev]) {
+  cudaMemPool_t& p = pools[id];
+  if (!p) {
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = dev;
-    cudaMemPool_t p = nullptr;
     e = cudaMemPoolCreate(&p, &props);
     unsigned long long keep = kPoolKeeps;
     if (e == cudaSuccess) e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-    if (e != cudaSuccess) return e;
-    pools[dev] = p;
+    if (e != cudaSuccess) {
+      if (p) cudaMemPoolDestroy(p);
+      pools.erase(id);
+      return e;
+    }
   }
-  *pool = pools[dev];
+  *pool = p;
   return cudaSuccess;
 }
 

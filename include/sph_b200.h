@@ -441,7 +441,8 @@ sph_status sph_mlp_features(sph_ctx* ctx, float* features, float* dlogh, uint32_
 /* The fraction of the run completed (the eighth input); read by the device at each step. */
 sph_status sph_set_progress(sph_ctx* ctx, float fraction);
 
-/* The network on its own, on the calling thread's current device (host arrays, blocking). */
+/* The network on its own, on the calling thread's current device (host arrays, blocking). These calls keep up to 64 MB of
+ * the device memory that they used for the next one, until the process or its device context ends. */
 typedef struct sph_mlp_train_cfg {
   uint32_t epochs;        /* passes over the samples */
   uint32_t batch;         /* samples per Adam step */

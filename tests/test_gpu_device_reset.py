@@ -1,6 +1,5 @@
-"""Calls without a context after a cudaDeviceReset, which ends the process's own device
-context: the library's kernels come back
-with their default limits, and every device pointer of before is gone.
+"""Calls without a context (allocation-free gravity, the MLP) after a cudaDeviceReset, which ends the process's own device
+context: the library's kernels come back with their default limits, and every device pointer and pool of before is gone.
 Each case runs in a process of its own, with buffers from the CUDA runtime, since a reset would take torch's along."""
 import subprocess
 import sys
@@ -50,6 +49,29 @@ GRAVITY = """
             assert np.array_equal(call(leaf), want)
 """
 
+MLP = """
+    def call():
+        rng = np.random.default_rng(6)
+        n = 700
+        p = rng.normal(scale=0.1, size=_lib.MLP_PARAMS).astype(np.float32)
+        p[-1], p[-10:-2] = 1.0, 1.0  # scales of the target and of the inputs
+        x, t = rng.normal(size=(n, 8)).astype(np.float32), rng.normal(size=n).astype(np.float32)
+        y, g, loss = np.empty(n, np.float32), np.empty(_lib.MLP_TRAINABLE, np.float32), np.empty(2, np.float32)
+        assert L.sph_mlp_forward(ptr(p), ptr(x), n, ptr(y)) == _lib.SPH_OK
+        assert L.sph_mlp_grad(ptr(p), ptr(x), ptr(t), n, ptr(g), ptr(loss)) == _lib.SPH_OK
+        cfg = _lib.MlpTrainCfg(epochs=2, batch=256, lr=1e-3, seed=3)
+        assert L.sph_mlp_train(ptr(p), ptr(x), ptr(t), n, C.byref(cfg), ptr(loss)) == _lib.SPH_OK
+        assert np.isfinite(y).all() and np.isfinite(g).all() and np.isfinite(p).all()
+        return y, g, p
+
+    want = call()
+    for _ in range(2):
+        ok(rt.cudaDeviceReset())
+        for a, b in zip(call(), want):
+            assert np.array_equal(a, b)
+"""
+
+
 def _run(case):
     r = subprocess.run([sys.executable, "-c", textwrap.dedent(PROLOGUE) + textwrap.dedent(case)], capture_output=True,
                        text=True, timeout=240)
@@ -58,3 +80,7 @@ def _run(case):
 
 def test_allocation_free_gravity_after_a_reset():
     _run(GRAVITY)
+
+
+def test_mlp_calls_after_a_reset():
+    _run(MLP)
