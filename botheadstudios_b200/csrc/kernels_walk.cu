@@ -594,8 +594,9 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
   // Sources in pairs, as in the far loop (their smoothing lengths in hs); every packed operation rounds as its scalar
   // form, so the distances and the predicate are those of the scalar loop below, source by source. A test is the sign
   // of d² − lim², shifted into `found`. The particle itself goes through the loop like any other source: at d = 0 its
-  // force is a finite number times zero (soft2 >= kNearSoft2), flush_p2p takes its bit and its potential back.
-  auto near_pairs = [&](auto loose) {
+  // force is a finite number times zero (soft2 >= kNearSoft2), flush_p2p takes its bit back. Its potential, which may be
+  // far larger than all others together, is left out by its place in the chunk (`self`, 32: not in it).
+  auto near_pairs = [&](auto loose, int self) {
     const float2 npx = make_float2(-pi.x, -pi.x), npy = make_float2(-pi.y, -pi.y), npz = make_float2(-pi.z, -pi.z);
     const float2 s2 = make_float2(soft2, soft2);
 #pragma unroll 2
@@ -633,7 +634,8 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
         fx2 = __ffma2_rn(g, dx, fx2);
         fy2 = __ffma2_rn(g, dy, fy2);
         fz2 = __ffma2_rn(g, dz, fz2);
-        if (OUT != kWalkAcc) fphi2 = __fadd2_rn(fphi2, make_float2(-gm.x, -gm.y));
+        if (OUT != kWalkAcc)
+          fphi2 = __fadd2_rn(fphi2, make_float2(self == 2 * k ? 0.0f : -gm.x, self == 2 * k + 1 ? 0.0f : -gm.y));
       }
     }
   };
@@ -734,13 +736,11 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
             if (NBR && skin > 0.0f) near_sources(std::true_type{});
             else near_sources(std::false_type{});
           } else {
-            if (NBR && skin > 0.0f) near_pairs(std::true_type{});
-            else near_pairs(std::false_type{});
+            const int self = OUT != kWalkAcc && holds_own ? place[lane] : 32;
+            if (NBR && skin > 0.0f) near_pairs(std::true_type{}, self);
+            else near_pairs(std::false_type{}, self);
           }
-          if (holds_own && place[lane] < 32) {
-            found &= ~(0x80000000u >> place[lane]);
-            if (GRAV && OUT != kWalkAcc && !one_by_one) phi += fmul(fmul(body[t].w, G), rsqrt_ftz(soft2));
-          }
+          if (holds_own && place[lane] < 32) found &= ~(0x80000000u >> place[lane]);
         }
       }
       if constexpr (NBR && F == 1) {
