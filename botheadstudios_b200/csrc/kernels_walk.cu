@@ -206,9 +206,6 @@ __device__ __forceinline__ void local_eval(const float cf[kLocal], float yx, flo
   }
 }
 
-// A particle meets itself in its own leaf: with soft2 above this, G m / soft2^1.5 stays finite for every G m below 3e20.
-constexpr float kNearSoft2 = 1.0e-12f;
-
 // What a gravity walk writes: the acceleration alone (a step's walk: the KDK integrator needs no potential),
 // the acceleration and the potential φ, or φ alone (into .w of the gravity record, for the energy diagnostic
 // of a state whose step walk left it out).
@@ -594,7 +591,7 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
   // Sources in pairs, as in the far loop (their smoothing lengths in hs); every packed operation rounds as its scalar
   // form, so the distances and the predicate are those of the scalar loop below, source by source. A test is the sign
   // of d² − lim², shifted into `found`. The particle itself goes through the loop like any other source: at d = 0 its
-  // force is a finite number times zero (soft2 >= kNearSoft2), flush_p2p takes its bit back. Its potential, which may be
+  // force is a finite number times zero (one_by_one), flush_p2p takes its bit back. Its potential, which may be
   // far larger than all others together, is left out by its place in the chunk (`self`, 32: not in it).
   auto near_pairs = [&](auto loose, int self) {
     const float2 npx = make_float2(-pi.x, -pi.x), npy = make_float2(-pi.y, -pi.y), npz = make_float2(-pi.z, -pi.z);
@@ -639,7 +636,7 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
       }
     }
   };
-  // One source at a time: hi/lo coordinates, and softenings too small for the particle's own term above.
+  // One source at a time: hi/lo coordinates, and particles whose own term above is not finite.
   auto near_sources = [&](auto loose) {
 #pragma unroll 4
     for (int k = 0; k < 32; ++k) {
@@ -687,7 +684,11 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
   // Rounds of F chunks, one for each warp; a particle's list takes the warps' finds in their order, so the list is
   // that of a single warp going through the chunks.
   constexpr unsigned kBatch = 4;
-  const bool one_by_one = HILO || (GRAV && soft2 < kNearSoft2);
+  bool one_by_one = HILO;
+  if (GRAV && !HILO) {  // a particle's own term in near_pairs, rounded as there: G m / soft³ (NaN without either)
+    const float rinv = rsqrt_ftz(soft2), own = fmul(fmul(fmul(fmul(body[tl].w, G), rinv), rinv), rinv);
+    one_by_one = __any_sync(SPH_FULL_MASK, !(fabsf(own) <= 3.4028235e38f));
+  }
   auto flush_p2p = [&](int count) {
     const int per = near_per;  // leaves per chunk
     float4 nsrc;

@@ -78,3 +78,12 @@ def test_a_batch_across_the_line_equals_each_impact_alone():
         for f in ("pos", "vel", "h", "u", "rho"):
             assert np.array_equal(state[f][a:b], one[f]), (k, f)
         assert np.array_equal(grav[a:b], g1)
+
+
+@pytest.mark.parametrize("n", [33, 1000, LINE + 1])
+def test_heavy_particles_with_a_small_softening(n):
+    """G m / soft³ beyond the f32 range: a particle's own (zero) force must not come out as infinity times zero."""
+    p = _cloud(n, 5, 2.2)
+    p["mass"] *= np.float32(1e30)
+    for soft in (1e-2, 1e-3, 1e-4):
+        _check(p, 16, 0, soft)
