@@ -101,6 +101,14 @@ struct Acc3 {
   }
 };
 
+// a += b; returns what the sum's rounding left out (Knuth's two-sum: either may be the larger).
+__device__ __forceinline__ float add_exact(float& a, float b) {
+  const float s = fadd(a, b), t = fsub(s, a);
+  const float e = fadd(fsub(a, fsub(s, t)), fsub(b, t));
+  a = s;
+  return e;
+}
+
 // ---- the group's local expansion --------------------------------------------------------------------------
 // An accepted node far from the group (|COM − z| >= r_g/θ_L, z the centre of the group's box and r_g its
 // half-diagonal) does not go through a per-particle multipole evaluation: its potential is expanded about z,
@@ -1088,10 +1096,12 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
   }  // parts
 
   if (GRAV) {
-    // the warps' sums in the warps' order
+    // the warps' sums in the warps' order (with hi/lo coordinates each with its compensation)
     if (!HILO) {
       acc.add<false>(fx2.x + fx2.y, fy2.x + fy2.y, fz2.x + fz2.y);
       phi += fphi2.x + fphi2.y;
+    } else if (F > 1) {
+      S.q0[w][lane] = make_float4(acc.cx, acc.cy, acc.cz, 0.0f);
     } else {
       acc.x -= acc.cx;
       acc.y -= acc.cy;
@@ -1116,13 +1126,27 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
   if (w != 0) return;
   if (in_group && GRAV) {
     float4 r = S.src[0][lane];
+    float4 c = make_float4(0.f, 0.f, 0.f, 0.f);  // what the sums are too large by
+    if constexpr (HILO && F > 1) c = S.q0[0][lane];
 #pragma unroll
     for (int k = 1; k < F; ++k) {
       const float4 v = S.src[k][lane];
-      r.x += v.x;
-      r.y += v.y;
-      r.z += v.z;
+      if constexpr (HILO) {
+        const float4 vc = S.q0[k][lane];
+        c.x += vc.x - add_exact(r.x, v.x);
+        c.y += vc.y - add_exact(r.y, v.y);
+        c.z += vc.z - add_exact(r.z, v.z);
+      } else {
+        r.x += v.x;
+        r.y += v.y;
+        r.z += v.z;
+      }
       r.w += v.w;
+    }
+    if constexpr (HILO && F > 1) {
+      r.x -= c.x;
+      r.y -= c.y;
+      r.z -= c.z;
     }
     if (OUT == kWalkPhi) reinterpret_cast<float*>(gout)[4 * (size_t)t + 3] = r.w;
     else gout[t] = make_float4(r.x, r.y, r.z, OUT == kWalkAccPhi ? r.w : 0.0f);
