@@ -3,10 +3,10 @@
 A batch of impacts of uneven size is split into size buckets, each tuned on its own; buckets whose tuned launch
 configurations agree share one context, which advances all of their impacts with one launch per phase (with one
 configuration for every bucket, the whole batch is one context), and contexts of different configurations run
-concurrently on their own streams. The autotuner picks, per bucket, the LBVH leaf size, the block size of the
-per-particle gather kernels (density, h-solve, forces) and the walk's tile (without effect: the walk chooses how
-many warps share a group by the impact's size) by timing candidates on a probe batch drawn from that bucket.
-Choices are cached in a JSON file keyed by the GPU name and the bucket.
+concurrently on their own streams. The autotuner picks, per bucket, the LBVH leaf size and the block size of the
+per-particle gather kernels (density, h-solve, forces) by timing candidates on a probe batch drawn from that bucket.
+Choices are cached in a JSON file keyed by the GPU name and the bucket. A choice also carries the walk's tile, which
+has no effect any more (the walk chooses how many warps share a group by the impact's size) and stays at its default.
 
 The reference has no counterpart: its offline driver runs impacts one after another
 (tools/impact-run/src/main.rs:645-671).
@@ -64,7 +64,9 @@ def _load_network(s, cfg: dict):
 
 class Autotuner:
     """Coordinate search over CANDIDATES (leaf size, then walk tile, then block size), each candidate timed on
-    the same probe batch: a fresh context, one warm-up step (the full rebuild), `steps` timed steps."""
+    the same probe batch: a fresh context, one warm-up step (the full rebuild), `steps` timed steps. The tile's
+    times differ by noise alone, so they are logged and not chosen by: buckets would end up in contexts of their
+    own for a tile that does nothing."""
 
     def __init__(self, base: dict, cache_path: str | None = None, steps: int = 2, device: int = -1):
         self.base = dict(base)
@@ -98,7 +100,7 @@ class Autotuner:
     def tune(self, bucket: int, probe: ic.Batch) -> dict:
         key = self._key(bucket)
         if key in self.cache:
-            return dict(self.cache[key])
+            return dict(self.cache[key], walk_warps=DEFAULT_CHOICE["walk_warps"])  # (older caches chose one)
         start = len(self.log)
         best = dict(DEFAULT_CHOICE)
         best_rate = self.measure(probe, best)
@@ -110,7 +112,7 @@ class Autotuner:
                     continue
                 timed.append(trial)
                 r = self.measure(probe, trial)
-                if r > best_rate:
+                if r > best_rate and name != "walk_warps":
                     best, best_rate = trial, r
         self.bucket_logs[bucket] = self.log[start:]
         self.cache[key] = best

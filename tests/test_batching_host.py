@@ -172,3 +172,13 @@ def test_tune_buckets_unifies_when_rates_tie(monkeypatch):
     monkeypatch.setattr(batching, "Autotuner", Fake)
     choices, _ = batching.tune_buckets(B, dict(kernel="wendland"))
     assert batching.context_groups(sorted(choices), choices) == [sorted(choices)]
+
+
+def test_autotuner_does_not_choose_a_walk_tile(tmp_path):
+    """The tile has no effect, so its times are noise: neither a lucky one nor one of an older cache is taken."""
+    cache = str(tmp_path / "tune.json")
+    t = _FakeTuner(lambda c: 100.0 + c["walk_warps"] + c["leaf_size"], cache_path=cache)
+    want = dict(leaf_size=32, walk_warps=2, block_threads=256)
+    assert t.tune(0, probe=None) == want
+    json.dump({"fake|bucket0": dict(want, walk_warps=8)}, open(cache, "w"))
+    assert _FakeTuner(lambda c: 1.0, cache_path=cache).tune(0, probe=None) == want
