@@ -4,7 +4,7 @@
 // cudaMalloc/cudaFree would synchronise the whole device and stall the frame, or a host engine whose device
 // memory is reserved up front by its own allocator and hands plug-ins only the buffers it owns. For them,
 // sph_gravity_tree_noalloc runs the same LBVH pipeline as the context path (bbox, Morton keys, radix sort,
-// Karras, moments, group-MAC walk) with every scratch buffer carved out of one fixed array in device
+// links and moments bottom-up, the point sets' walk) with every scratch buffer carved out of one fixed array in device
 // memory, compiled into the library. The caller passes device pointers for the input points and the output
 // accelerations. The array holds at most kNoAllocMaxPoints points; every GPU that loads the library keeps it
 // for the life of the process.
@@ -190,18 +190,8 @@ Dev carve_dev(unsigned char* base, uint32_t K) {
   return d;
 }
 
-// Everything the walk reads from DevParams, written on the device (no host copy), counters cleared; the segment table. And
-// what the sort and the tree keep in the scratch between calls, as they leave it at their end: calls that overlapped in
-// spite of the interface spoil each other's results, but not those of the calls after them. (The sort's epoch goes on: words
-// that an overlapped sort published carry an older one.)
-__global__ void __launch_bounds__(1024) k_noalloc_params(DevParams* P, Seg* segs, int n, int L, float soft2, float G,
-                                                         float theta, SortCtl* sort, unsigned long long* slots) {
-  for (int k = threadIdx.x; k < SO_PASSES * SO_BINS; k += blockDim.x) (&sort->hist[0][0])[k] = 0u;
-  for (int k = threadIdx.x; k < L; k += blockDim.x) slots[k] = 0ull;
-  if (threadIdx.x <= SO_PASSES) sort->done[threadIdx.x] = 0u;
-  if (threadIdx.x != 0) return;
-  sort->ticket = sort->finished = 0u;
-  ++sort->end.epoch;
+// Everything the walk reads from DevParams, written on the device (no host copy), counters cleared; the segment table.
+__global__ void k_noalloc_params(DevParams* P, Seg* segs, int n, int L, float soft2, float G, float theta) {
   DevParams p;
   memset(&p, 0, sizeof(p));
   p.G = G;
@@ -211,9 +201,19 @@ __global__ void __launch_bounds__(1024) k_noalloc_params(DevParams* P, Seg* segs
 }
 
 // The points and their bounding box (three launches fewer than with a reset, a box and a segment kernel of their own:
-// 16,001 points 263 µs instead of 273).
-__global__ void __launch_bounds__(256) k_noalloc_load(const float4* __restrict__ in, int n, State st, Seg* segs) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// 16,001 points 263 µs instead of 273). And what the sort and the tree keep in the scratch between calls, as they leave it
+// at their end: calls that overlapped in spite of the interface spoil each other's results, but not those of the calls after
+// them. (The sort's epoch goes on: words that an overlapped sort published carry an older one.)
+__global__ void __launch_bounds__(256) k_noalloc_load(const float4* __restrict__ in, int n, State st, Seg* segs, int L,
+                                                      SortCtl* sort, unsigned long long* slots) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
+  for (int k = i; k < SO_PASSES * SO_BINS; k += threads) (&sort->hist[0][0])[k] = 0u;
+  for (int k = i; k < L; k += threads) slots[k] = 0ull;
+  if (i <= SO_PASSES) sort->done[i] = 0u;
+  if (i == 0) {
+    sort->ticket = sort->finished = 0u;
+    ++sort->end.epoch;
+  }
   unsigned lo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, hi[3] = {0u, 0u, 0u};
   if (i < n) {
     const float4 b = in[i];
@@ -276,9 +276,9 @@ extern "C" sph_status sph_gravity_tree_noalloc(const void* d_bodies4, uint32_t n
   c.quad = (int)multipole;
   c.mac = SPH_MAC_GROUP;
   c.local_theta = kLocalThetaDefault;  // the walk sph_gravity runs with the default configuration
-  k_noalloc_params<<<1, 1024, 0, s>>>(d.P, d.segs, d.n, d.L, softening * softening, (float)G, theta,
-                                      static_cast<SortCtl*>(d.sort_work), d.slots);
-  k_noalloc_load<<<(n + 255) / 256, 256, 0, s>>>(static_cast<const float4*>(d_bodies4), (int)n, d.st[0], d.segs);
+  k_noalloc_params<<<1, 1, 0, s>>>(d.P, d.segs, d.n, d.L, softening * softening, (float)G, theta);
+  k_noalloc_load<<<(n + 255) / 256, 256, 0, s>>>(static_cast<const float4*>(d_bodies4), (int)n, d.st[0], d.segs, d.L,
+                                                   static_cast<SortCtl*>(d.sort_work), d.slots);
   launch_segments(d, s);
   launch_sort_permute(d, false, s);
   launch_tree(d, c, theta, s);
