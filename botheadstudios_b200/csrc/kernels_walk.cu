@@ -601,7 +601,7 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
   // of d² − lim², shifted into `found`. The particle itself goes through the loop like any other source: at d = 0 its
   // force is a finite number times zero (one_by_one), flush_p2p takes its bit back. Its potential, which may be
   // far larger than all others together, is left out by its place in the chunk (`self`, 32: not in it).
-  auto near_pairs = [&](auto loose, int self) {
+  auto near_pairs = [&](auto loose, auto own, int self) {
     const float2 npx = make_float2(-pi.x, -pi.x), npy = make_float2(-pi.y, -pi.y), npz = make_float2(-pi.z, -pi.z);
     const float2 s2 = make_float2(soft2, soft2);
 #pragma unroll 2
@@ -639,8 +639,10 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
         fx2 = __ffma2_rn(g, dx, fx2);
         fy2 = __ffma2_rn(g, dy, fy2);
         fz2 = __ffma2_rn(g, dz, fz2);
-        if (OUT != kWalkAcc)
+        if constexpr (OUT != kWalkAcc && decltype(own)::value)
           fphi2 = __fadd2_rn(fphi2, make_float2(self == 2 * k ? 0.0f : -gm.x, self == 2 * k + 1 ? 0.0f : -gm.y));
+        else if (OUT != kWalkAcc)
+          fphi2 = __fadd2_rn(fphi2, make_float2(-gm.x, -gm.y));
       }
     }
   };
@@ -745,9 +747,13 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
             if (NBR && skin > 0.0f) near_sources(std::true_type{});
             else near_sources(std::false_type{});
           } else {
-            const int self = OUT != kWalkAcc && holds_own ? place[lane] : 32;
-            if (NBR && skin > 0.0f) near_pairs(std::true_type{}, self);
-            else near_pairs(std::false_type{}, self);
+            if (OUT != kWalkAcc && holds_own) {  // one chunk or two of a group
+              if (NBR && skin > 0.0f) near_pairs(std::true_type{}, std::true_type{}, place[lane]);
+              else near_pairs(std::false_type{}, std::true_type{}, place[lane]);
+            } else {
+              if (NBR && skin > 0.0f) near_pairs(std::true_type{}, std::false_type{}, 32);
+              else near_pairs(std::false_type{}, std::false_type{}, 32);
+            }
           }
           if (holds_own && place[lane] < 32) found &= ~(0x80000000u >> place[lane]);
         }
