@@ -173,10 +173,12 @@ __global__ void k_density_eos(int n, State st, const unsigned* __restrict__ nbr,
   fdata[t] = eos_record(eos, st.mat[t], st.mass[t], r_i, st.vel_u[t].w, P);
 }
 
-// Lanes a particle takes in the density sums (measured while a list's entries lay in rows of one). The density of 10,240
-// particles 10.7 µs with four lanes, 12.8 with two (14.0 with one); a solve of two passes and the density 61 and 59 (62)
-// at 32,768, 145 and 135 (142) at 180,000, 656 and 562 (512) at 1,048,576 by itself, but with three contexts at once the
-// step there is shorter with two than with one (5,895 and 5,960).
+// Lanes a particle takes in the density sums. A solve of two passes and the density, four lanes and two (and one, while a
+// list's entries lay in rows of one): 28 and 30 µs (54, with more launches) at 5,000 particles, 30 and 31 (54) at 10,240,
+// 31 and 32 (56) at 15,000, 33.0 and 33.2 (57) at 20,000, 38 and 34 (57) at 32,768, 53 and 51 (65) at 65,536, 99 and 96
+// (118) at 180,000, 490 and 430 (409) at 1,048,576, 919 and 797 (734) at 2,000,000. One lane would round otherwise than
+// two and four, which give the same bits, so it is left to the learned runs; the step with three contexts at once was
+// shorter with two lanes than with one at 1,048,576 too (5,895 and 5,960).
 static int density_lanes(int n) { return n <= 20000 ? 4 : 2; }
 static int gather_blocks(int n, int blk, int lanes) { return (n + blk / lanes - 1) / (blk / lanes); }
 

@@ -411,7 +411,7 @@ uint32_t sph_dem_count(const sph_dem* dem);
  * device context (and the first after a cudaDeviceReset) looks up that array's device address; make that
  * first call before any stream capture (a first call inside a capture returns SPH_ERR_STATE). Every call
  * uses the same array, so calls whose work overlaps on the GPU (different streams, or different host threads
- * on one device) race and corrupt each other's results: order them on one stream. If the traversal stack
+ * on one device) race and corrupt each other's results (not those of later calls): order them on one stream. If the traversal stack
  * (4,096 nodes for 32 points) overflows, every output is NaN. A CUDA error already pending on the calling thread
  * is left in place and returns SPH_ERR_CUDA before any work is enqueued. */
 sph_status sph_gravity_tree_noalloc(const void* d_bodies4, uint32_t n, double G, float softening, float theta,
