@@ -294,10 +294,15 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
   const unsigned leaf0 = (unsigned)(L - 1);
   const unsigned lt = (1u << lane) - 1u;
   // staging of the pairwise lists: entries of K (near) or K/2 (far, when far leaves are split into halves)
-  // sources, 32/K entries per 32-source chunk; K is a power of two in the group walk, so shifts, not divisions
+  // sources, 32/K entries per 32-source chunk; K is a power of two in the group walk, so shifts, not divisions. The
+  // lists alone (PARTICLE mode has a gravity walk of its own) take any K <= 32: there a place in a chunk is divided by K
+  // through 1/K in 1,024ths, exact below 32
   const int ksh = 31 - __clz(K);
   const int kfsh = half > 0 ? ksh - 1 : ksh;
-  const int near_per = 32 >> ksh, near_li = (int)lane >> ksh, near_off = (int)lane & (K - 1);
+  const int kinv = GRAV ? 0 : (1023 + K) / K;
+  const auto leaf_of = [&](int k) { return GRAV ? k >> ksh : k * kinv >> 10; };
+  const auto place_of = [&](int k) { return GRAV ? k & (K - 1) : k - (k * kinv >> 10) * K; };
+  const int near_per = GRAV ? 32 >> ksh : 32 / K, near_li = leaf_of((int)lane), near_off = place_of((int)lane);
   const int far_per = 32 >> kfsh, far_li = (int)lane >> kfsh, far_off = (int)lane & ((1 << kfsh) - 1);
 
   Acc3 acc;
@@ -712,7 +717,7 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
       const int sidx = nidx;
       found = 0u;
       if (mine < count) {  // (the warp)
-        part_p2p += (unsigned)min(per, count - mine) << ksh;
+        part_p2p += GRAV ? (unsigned)min(per, count - mine) << ksh : (unsigned)(min(per, count - mine) * K);
         part_src += __popc(__ballot_sync(SPH_FULL_MASK, sidx >= 0));
         nidx = near_source(mine + per * F, count, nsrc, nh);
         src.w *= G;
@@ -779,7 +784,7 @@ __global__ void __launch_bounds__(F * 32, TW_WARPS_PER_SM / F) k_tree_walk(
             }
             const int k = __clz(m);
             m &= ~(0x80000000u >> k);
-            *out = (e[k >> ksh] >> 5) + (unsigned)(k & (K - 1));
+            *out = (e[leaf_of(k)] >> 5) + (unsigned)place_of(k);
             // the next entry of the row, or the next row's first
             out += (reinterpret_cast<uintptr_t>(out) & 12u) == 12u ? 125 : 1;
           }

@@ -87,3 +87,16 @@ def test_heavy_particles_with_a_small_softening(n):
     p["mass"] *= np.float32(1e30)
     for soft in (1e-2, 1e-3, 1e-4):
         _check(p, 16, 0, soft)
+
+
+@pytest.mark.parametrize("K", [1, 2, 3, 5, 7, 11, 12, 16, 17, 24, 31, 32])
+@pytest.mark.parametrize("n", [1, 100, 2000, LINE + 1])
+def test_neighbours_of_the_per_particle_mode_in_leaves_of_any_size(K, n):
+    p = _cloud(n, n + K, 2.2)
+    with GpuSph(n, G=1.0, leaf_size=K, mac=1, max_neighbours=256) as s:
+        s.upload(p, M.eos_table(), 0.1)
+        s.eval_forces()
+        assert s.diag()["overflow_flags"] == 0
+        nb = s.neighbour_sets()
+    want = oracle.neighbours32(np.concatenate([p["pos"], p["h"][:, None]], 1), cap=256)
+    assert all(np.array_equal(nb[i], want[i]) for i in range(n))
